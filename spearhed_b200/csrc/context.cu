@@ -681,7 +681,8 @@ int sph_ctx::allocate()
     dc.nPartialBlocks = sph::partialBlocks(n);
     if((st = alloc(dc.partials, size_t(dc.nPartialBlocks) * sph::kDiagWords))
        || (st = alloc(boxOut, size_t(nbox) * sph::kDiagWords))
-       || (st = alloc(boxScratch, sph::boxReduceScratchDoubles(nbox))) || (st = alloc(dc.lists.count, n)))
+       || (st = alloc(boxScratch, sph::boxReduceScratchDoubles(nbox))) || (st = alloc(dc.lists.count, n))
+       || (st = alloc(dc.lists.rowLen, n)))
         return st;
     SPH_CUDA_TRY(cudaMemsetAsync(dc.diag, 0, sizeof(double) * sph::kDiagWords, stream));
     dc.keyBits = 1;
@@ -791,7 +792,7 @@ int sph_ctx::probeListCapacity()
         int st = clearStatus();
         if(st || (st = build(false)))
             return st;
-        sph::launchDensity(dc, pa, p.kernel, p.precision, true, densityVariant, stream);
+        sph::launchNeighbours(dc, pa, p.precision, true, densityVariant, stream);
         uint32_t stat[sph::kStatWords];
         SPH_CUDA_TRY(cudaMemcpyAsync(stat, dc.status, sizeof(stat), cudaMemcpyDeviceToHost, stream));
         SPH_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -810,7 +811,7 @@ int sph_ctx::growLists(uint32_t need, bool bestEffort)
     {
         // headroom only: the new rows are allocated beside the old ones, and a
         // context that cannot have them keeps the lists it has
-        if(alloc(list, size_t(n) * capN) != SPH_OK)
+        if(alloc(list, size_t(n) * capN + sph::kRowSlack) != SPH_OK)
         {
             cudaGetLastError();
             return SPH_OK;
@@ -828,7 +829,7 @@ int sph_ctx::growLists(uint32_t need, bool bestEffort)
     }
     if(!list)
     {
-        int const st = alloc(list, size_t(n) * capN);
+        int const st = alloc(list, size_t(n) * capN + sph::kRowSlack);
         if(st)
             return st;
     }
@@ -890,7 +891,9 @@ int sph_ctx::densityPass()
 {
     sph::NvtxRange const range("density pass");
     SPH_CUDA_TRY(cudaMemsetAsync(dc.lists.count, 0xff, size_t(n) * 4, stream));
-    sph::launchDensity(dc, pa, p.kernel, p.precision, false, densityVariant, stream);
+    SPH_CUDA_TRY(cudaMemsetAsync(dc.lists.rowLen, 0, size_t(n) * 4, stream));
+    sph::launchNeighbours(dc, pa, p.precision, false, densityVariant, stream);
+    sph::launchDensity(dc, pa, p.kernel, p.precision, stream);
     return SPH_OK;
 }
 

@@ -161,12 +161,16 @@ namespace sph
         uint32_t* bend;
     };
 
-    //! Neighbour lists: row t (sorted target index) holds count[t] entries of
-    //! packEntry(j, stencil slot) at list[t * cap + k].
+    //! Neighbour lists: row t (sorted target index) starts at list[t * cap] and
+    //! holds rowLen[t] entries packEntry(j, stencil slot).
+    //! The pair passes load rows in groups of 16 entries: the last row's group
+    //! may reach this far past the array's end.
+    constexpr uint32_t kRowSlack = 16;
     struct Lists
     {
         uint32_t* list;
         uint32_t* count;
+        uint32_t* rowLen; //!< entries of the row the pair passes read (0 for rows not built)
         uint32_t cap;
     };
 
@@ -369,21 +373,25 @@ namespace sph
     uint32_t partialBlocks(uint32_t n);
 
     // ---- pair_kernels.cu
-    //! Neighbour build + density (+ records for the force pass); countOnly only counts.
-    //! Pair-kernel launches; `variant` picks the launch shape (0 = default,
-    //! see densityVariants / forceVariants).
-    void launchDensity(
+    // ---- neighbours.cu
+    //! Accepted-pair counts and list rows of the current cells; countOnly only
+    //! counts.  `variant` picks the launch shape (0 = default, densityVariants).
+    void launchNeighbours(
         DevCtx const& c,
         PhysArgs const& pa,
-        int kernel,
         int precision,
         bool countOnly,
         int variant,
         cudaStream_t s);
-    void launchForce(DevCtx const& c, PhysArgs const& pa, int kernel, int precision, int variant, cudaStream_t s);
     int densityVariants(int precision);
-    int forceVariants(int precision);
     void densityShape(int precision, int variant, int* stagingDepth, int* blocksPerSm, int* cullUnroll);
+    void configureNeighbourKernels();
+
+    // ---- pair_kernels.cu
+    //! Density sum over the rows, and the records of the force pass.
+    void launchDensity(DevCtx const& c, PhysArgs const& pa, int kernel, int precision, cudaStream_t s);
+    void launchForce(DevCtx const& c, PhysArgs const& pa, int kernel, int precision, int variant, cudaStream_t s);
+    int forceVariants(int precision);
     int forceBlocksPerSm(int precision, int physics, int variant);
     //! Sets the shared-memory attributes of every pair-kernel instantiation
     //! (once, before any launch, so no attribute call happens during a graph capture).
