@@ -306,6 +306,29 @@ namespace sph
             }
         }
 
+        //! Warps per cell, as a power of two: a cell's targets are dealt to 2^shift
+        //! warps in groups of 64 >> shift.  A group shares its staged windows, so
+        //! large groups cost least work, but few particles in groups of 64 leave
+        //! most warps idle behind the cells with the longest stencils: the group
+        //! halves until n / group fills the resident warps 1.25 times.  Density
+        //! pass at groups of 64 / 32 / 16 / 8 / 4, ms: FP64 Sod 2.3 k 0.195 / 0.147 /
+        //! 0.116 / 0.102 / 0.098; FP32 Sod 18 k 0.167 / 0.136 / 0.135 / 0.130 / 0.128;
+        //! FP64 Brio-Wu 176 k 0.349 / 0.316 / 0.337 / 0.426 / 0.639; FP64 Orszag-Tang
+        //! 206 k 0.306 / 0.323 / 0.354 / 0.453 / 0.651; FP32 Brio-Wu 2 M 1.37 / 1.56 /
+        //! 1.82 / 2.60 / 4.35.  Grids with many more cells than particles are not
+        //! split (each part asks for the cell's range).  The rows are the same for
+        //! every group: a target's entries keep their candidate order.
+        constexpr int kMaxPartShift = 4;
+        __device__ __forceinline__ int partsShift(uint32_t n, uint32_t cells, uint32_t warps)
+        {
+            int s = 0;
+            while(s < kMaxPartShift && uint64_t(n) * 4u < uint64_t(warps) * 5u * (64u >> s))
+                ++s;
+            while(s > 0 && (uint64_t(cells) << s) > 16ull * n)
+                --s;
+            return s;
+        }
+
         //! Tunable launch shapes (picked per context by sph_autotune): CAP is the
         //! staging depth (candidates per shared-memory window), MINB the blocks
         //! per SM the register allocation must admit, CU the unroll depth of the
@@ -346,7 +369,10 @@ namespace sph
             // takes its next item from a counter; the fetch for the next item is
             // issued first and read at the loop's end.  Item q is cell
             // q - activeBase of the box whose range holds it.
-            uint32_t const nWork = *c.activeTotal;
+            int const partShift = partsShift(c.n, *c.activeTotal, 148u * uint32_t(MINB) * kWarps);
+            uint32_t const group = 64u >> partShift;
+            uint32_t const parts = 1u << partShift;
+            uint32_t const nWork = *c.activeTotal << partShift;
             uint32_t pending = 0;
             if(lane == 0)
                 pending = atomicAdd(c.work, 1u);
@@ -354,16 +380,19 @@ namespace sph
             {
                 if(lane == 0)
                     pending = atomicAdd(c.work, 1u);
-                int const box = boxOfWork(c.boxes, c.nbox, q);
+                uint32_t const item = q >> partShift;
+                int const box = boxOfWork(c.boxes, c.nbox, item);
                 // item -> cell: the box's level-0 cells first, then its level-1 cells
-                uint32_t const l = q - c.boxes[box].activeBase;
+                uint32_t const l = item - c.boxes[box].activeBase;
                 uint32_t const nc0 = c.boxes[box].ncells;
                 uint32_t const cell = c.boxes[box].cellBase + (l < nc0 ? l : c.boxes[box].ncellsMax + (l - nc0));
                 if(!checkIndex(cell < c.cells.ncells, c.status, kChkCell))
                     continue;
                 uint32_t const tBeg = c.cells.start[cell];
                 uint32_t const tEnd = c.cells.mid[cell];
-                if(tBeg >= tEnd || !checkIndex(tEnd <= c.n, c.status, kChkTargets))
+                // this part's first targets; the parts of a cell take groups in turn
+                uint32_t const tFirst = tBeg + (q & (parts - 1u)) * group;
+                if(tFirst >= tEnd || !checkIndex(tEnd <= c.n, c.status, kChkTargets))
                     continue;
                 BoxDev const& B = c.boxes[box];
                 // Target cell: level 0 (the grid) or level 1 (one of the m0 x m1 x m2
@@ -504,15 +533,15 @@ namespace sph
                 describe(lane, sBeg0, sCnt0, slot0, sh0);
                 scan(sCnt0, pre0, total0);
 
-                // Two target chunks (up to 64 targets) share every staged window.
-                for(uint32_t tc = tBeg; tc < tEnd; tc += 64)
+                // Two target chunks (a group of up to 64 targets) share every staged window.
+                for(uint32_t tc = tFirst; tc < tEnd; tc += group << partShift)
                 {
                     TargetChunk<T> A, Bc;
-                    uint32_t const ntA = min(32u, tEnd - tc);
-                    uint32_t const ntB = tc + 32 < tEnd ? min(32u, tEnd - tc - 32) : 0u;
+                    uint32_t const nTargets = min(group, tEnd - tc);
+                    uint32_t const ntA = min(32u, nTargets);
+                    uint32_t const ntB = nTargets - ntA;
                     initChunk(A, rec, tc, ntA, lane, supT);
                     initChunk(Bc, rec, tc + 32, ntB, lane, supT);
-                    uint32_t const nTargets = ntA + ntB;
                     // Bounding box of the two chunks' targets and their largest cull
                     // radius: staging keeps only candidates within that radius of the
                     // box.  For a target x_i in [lo, hi] and a staged -x_j, rounding
@@ -753,9 +782,9 @@ namespace sph
             size_t const smem = neighbourSmem<T, PM, CAP>();
             // persistent grid: enough resident blocks to fill every SM; cells come
             // from the work queue
-            uint32_t blocks = (c.cells.ncells + kWarps - 1) / kWarps;
             uint32_t const resident = 148u * uint32_t(MINB);
-            blocks = blocks > resident ? resident : blocks;
+            uint64_t const items = (uint64_t(c.cells.ncells) << kMaxPartShift) / kWarps + 1;
+            uint32_t const blocks = items > resident ? resident : uint32_t(items);
             if(blocks)
             {
                 cudaMemsetAsync(c.work, 0, sizeof(uint32_t), s);
