@@ -664,7 +664,7 @@ int sph_ctx::allocate()
             return st;
     }
     dc.cells.ncells = ncells;
-    if((st = alloc(dc.cells.start, ncells)) || (st = alloc(dc.cells.mid, ncells)) || (st = alloc(dc.cells.end, ncells))
+    if((st = alloc(dc.cells.start, size_t(ncells) * 3))
        || (st = alloc(dc.cells.bstart, ncells)) || (st = alloc(dc.cells.bend, ncells)))
         return st;
     if((st = alloc(dc.keysA, n)) || (st = alloc(dc.valsA, n)) || (st = alloc(dc.keysB, n)) || (st = alloc(dc.valsB, n))
@@ -684,6 +684,8 @@ int sph_ctx::allocate()
        || (st = alloc(boxScratch, sph::boxReduceScratchDoubles(nbox))) || (st = alloc(dc.lists.count, n))
        || (st = alloc(dc.lists.rowLen, n)))
         return st;
+    dc.cells.mid = dc.cells.start + ncells;
+    dc.cells.end = dc.cells.mid + ncells;
     SPH_CUDA_TRY(cudaMemsetAsync(dc.diag, 0, sizeof(double) * sph::kDiagWords, stream));
     dc.keyBits = 1;
     while((uint64_t(1) << dc.keyBits) <= uint64_t(ncells) * 2)
@@ -750,6 +752,8 @@ int sph_ctx::uploadMirror()
     SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.time, 0, 8 * dts.size(), stream));
     SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.lastDt, 0, 8 * dts.size(), stream));
     SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.chBits, 0, 8 * dts.size(), stream));
+    SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.hmaxBits, 0, 8 * dts.size(), stream));
+    SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.hminBits, 0xff, 8 * dts.size(), stream));
     SPH_CUDA_TRY(cudaStreamSynchronize(stream));
     mirrorStale = false;
     deviceCurrent = true;
@@ -869,9 +873,6 @@ int sph_ctx::ensureDevice()
 int sph_ctx::build(bool drift)
 {
     sph::NvtxRange const range(drift ? "drift + cell sort" : "cell sort");
-    SPH_CUDA_TRY(cudaMemsetAsync(&dc.scal->pairs, 0, sizeof(unsigned long long), stream));
-    SPH_CUDA_TRY(cudaMemsetAsync(&dc.scal->candidates, 0, sizeof(unsigned long long), stream));
-    SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.chBits, 0, sizeof(unsigned long long) * dc.nbox, stream));
     if(p.cull == SPH_CULL_PAIR_MAX)
         sph::launchGridUpdate(dc, supportOf(p.kernel), stream);
     sph::launchDriftKeys(dc, drift, stream);
@@ -890,8 +891,6 @@ int sph_ctx::build(bool drift)
 int sph_ctx::densityPass()
 {
     sph::NvtxRange const range("density pass");
-    SPH_CUDA_TRY(cudaMemsetAsync(dc.lists.count, 0xff, size_t(n) * 4, stream));
-    SPH_CUDA_TRY(cudaMemsetAsync(dc.lists.rowLen, 0, size_t(n) * 4, stream));
     sph::launchNeighbours(dc, pa, p.precision, false, densityVariant, stream);
     sph::launchDensity(dc, pa, p.kernel, p.precision, stream);
     return SPH_OK;
@@ -900,7 +899,6 @@ int sph_ctx::densityPass()
 int sph_ctx::forcePass()
 {
     sph::NvtxRange const range("force pass");
-    SPH_CUDA_TRY(cudaMemsetAsync(dc.bs.dtBits, 0x7f, sizeof(unsigned long long) * dc.nbox, stream));
     sph::launchForce(dc, pa, p.kernel, p.precision, forceVariant, stream);
     return SPH_OK;
 }

@@ -787,7 +787,6 @@ namespace sph
             uint32_t const blocks = items > resident ? resident : uint32_t(items);
             if(blocks)
             {
-                cudaMemsetAsync(c.work, 0, sizeof(uint32_t), s);
                 kNeighbours<T, PM, CAP, MINB, CU><<<blocks, kWarps * 32, smem, s>>>(c, pa.h0, countOnly);
                 countLaunches(1);
             }

@@ -420,9 +420,9 @@ int sph_density_noalloc(
     uint32_t* sortScr = cv.take<uint32_t>(sph::radixScratchWords(nn));
     sph::Cells cells{};
     cells.ncells = uint32_t(ncells);
-    cells.start = cv.take<uint32_t>(ncells);
-    cells.mid = cv.take<uint32_t>(ncells);
-    cells.end = cv.take<uint32_t>(ncells);
+    cells.start = cv.take<uint32_t>(3 * ncells); // one array, see Cells
+    cells.mid = cells.start + ncells;
+    cells.end = cells.mid + ncells;
     sph::D4* pm64 = nullptr;
     double* hc64 = nullptr;
     float4* pm32 = nullptr;

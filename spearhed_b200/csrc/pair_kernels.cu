@@ -151,6 +151,8 @@ namespace sph
             constexpr int S = kLanes<T>;
             uint32_t const sub = threadIdx.x & uint32_t(S - 1);
             uint32_t const t = (blockIdx.x * kThreads + threadIdx.x) / S;
+            if(blockIdx.x == 0 && threadIdx.x == 0)
+                *c.work = 0; // the neighbour build's queue, should it run again on these cells
             bool const act = t < c.n && isTarget(c.cur.role[t]);
             int const myBox = act ? c.cur.box[t] : -1;
             Acc<T> rho;

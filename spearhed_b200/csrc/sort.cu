@@ -6,12 +6,18 @@
 // particles are re-binned every step by a stable LSD radix sort on their cell
 // key, with no host round trip.
 //
-// Layout: one pass per 8-bit digit.  A pass is (1) a per-tile digit histogram,
-// (2) an exclusive scan of the digit-major [digit][tile] count table, (3) a
+// Layout: one pass per 8-bit digit, tiles of 256 x rounds keys.  A pass is (1) a
+// per-tile digit histogram, (2) the tiles' exclusive prefix per digit, (3) a
 // stable scatter: every tile ranks its keys per digit in input order (warp
 // __match_any_sync ranks, then a per-digit prefix over the warps of the block)
-// and writes them at the scanned offset.  Tiles are 4096 keys (256 threads x
-// 16 rounds); keys are read coalesced, once per kernel.
+// and writes them at the digit's base plus its tile's prefix.  Keys are read
+// coalesced, once per kernel.
+//
+// A pass is bound by latency and launches, not by its bytes (8 B in, 8 B out per
+// key): tiles of a fixed 4096 keys gave 18 k keys 5 blocks (10 us a histogram,
+// 12 us a scatter).  rounds follows the key count, for about 128 tiles up to half
+// a million keys and 16 rounds beyond; with up to kFewTiles tiles the scatter
+// adds the tiles' counts itself and step (2) needs no launch.
 #include "sph_launch.hpp"
 
 namespace sph
@@ -19,31 +25,92 @@ namespace sph
     namespace
     {
         constexpr int kThreads = 256;
-        constexpr int kRounds = 16;
-        constexpr int kTile = kThreads * kRounds;
+        constexpr uint32_t kMaxRounds = 16;
+        constexpr uint32_t kFewTiles = 192;
+
+        uint32_t tileRounds(uint32_t n)
+        {
+            uint32_t const r = n / (128u * kThreads);
+            return r < 1u ? 1u : (r > kMaxRounds ? kMaxRounds : r);
+        }
+        uint32_t tileCount(uint32_t n)
+        {
+            uint32_t const tile = kThreads * tileRounds(n);
+            return (n + tile - 1) / tile;
+        }
+
         constexpr int kScanItems = 8;
         constexpr int kScanTile = kThreads * kScanItems;
 
+        //! Digit counts of each tile, at tileHist[digit * ntile + tile], or with few
+        //! tiles at tileHist[tile * 256 + digit].  Keys come nearly sorted (the
+        //! order of the last step), so a warp's equal digits are counted once.
         __global__ void __launch_bounds__(kThreads) kRadixHist(
             uint32_t const* __restrict__ keys,
             uint32_t n,
             int shift,
+            uint32_t rounds,
             uint32_t* __restrict__ tileHist,
-            uint32_t ntile)
+            uint32_t ntile,
+            bool few)
         {
             __shared__ uint32_t h[256];
             h[threadIdx.x] = 0;
             __syncthreads();
-            uint32_t const base = blockIdx.x * uint32_t(kTile);
+            int const lane = threadIdx.x & 31;
+            uint32_t const base = blockIdx.x * uint32_t(kThreads) * rounds;
 #pragma unroll 4
-            for(int r = 0; r < kRounds; ++r)
+            for(uint32_t r = 0; r < rounds; ++r)
             {
-                uint32_t const i = base + uint32_t(r) * kThreads + threadIdx.x;
-                if(i < n)
-                    atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+                uint32_t const i = base + r * kThreads + threadIdx.x;
+                bool const valid = i < n;
+                uint32_t const digit = valid ? (keys[i] >> shift) & 255u : 0x100u;
+                uint32_t const peers = __match_any_sync(0xffffffffu, digit);
+                if(valid && (peers & ((1u << lane) - 1u)) == 0u)
+                    atomicAdd(&h[digit], uint32_t(__popc(peers)));
             }
             __syncthreads();
-            tileHist[threadIdx.x * ntile + blockIdx.x] = h[threadIdx.x];
+            tileHist[few ? blockIdx.x * 256u + threadIdx.x : threadIdx.x * ntile + blockIdx.x] = h[threadIdx.x];
+        }
+
+        //! Exclusive prefix over the tiles of digit blockIdx.x, in place, and the
+        //! digit's total.
+        __global__ void __launch_bounds__(kThreads)
+            kRadixRows(uint32_t* __restrict__ tileHist, uint32_t ntile, uint32_t* __restrict__ totals)
+        {
+            __shared__ uint32_t warpTot[kThreads / 32];
+            int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            uint32_t* const row = tileHist + size_t(blockIdx.x) * ntile;
+            uint32_t carry = 0;
+            for(uint32_t t0 = 0; t0 < ntile; t0 += kThreads)
+            {
+                uint32_t const t = t0 + threadIdx.x;
+                uint32_t const v = t < ntile ? row[t] : 0u;
+                uint32_t incl = v;
+#pragma unroll
+                for(int d = 1; d < 32; d <<= 1)
+                {
+                    uint32_t const o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if(lane >= d)
+                        incl += o;
+                }
+                if(lane == 31)
+                    warpTot[warp] = incl;
+                __syncthreads();
+                uint32_t before = carry;
+#pragma unroll
+                for(int w = 0; w < kThreads / 32; ++w)
+                {
+                    if(w < warp)
+                        before += warpTot[w];
+                    carry += warpTot[w];
+                }
+                if(t < ntile)
+                    row[t] = before + incl - v;
+                __syncthreads();
+            }
+            if(threadIdx.x == 0)
+                totals[blockIdx.x] = carry;
         }
 
         __global__ void __launch_bounds__(kThreads) kRadixScatter(
@@ -53,23 +120,60 @@ namespace sph
             uint32_t* __restrict__ valsOut,
             uint32_t n,
             int shift,
-            uint32_t const* __restrict__ tileOffset,
-            uint32_t ntile)
+            uint32_t rounds,
+            uint32_t const* __restrict__ tileHist,
+            uint32_t const* __restrict__ totals,
+            uint32_t ntile,
+            bool few)
         {
             __shared__ uint32_t running[256];
             __shared__ uint32_t warpCnt[kThreads / 32][256];
             int const tid = threadIdx.x;
             int const warp = tid >> 5;
             int const lane = tid & 31;
-            running[tid] = tileOffset[tid * ntile + blockIdx.x];
+            {
+                // digit tid: the tiles before this one, and all keys of the digit
+                uint32_t before = 0, total = 0;
+                if(few)
+                {
+#pragma unroll 8
+                    for(uint32_t t = 0; t < ntile; ++t)
+                    {
+                        uint32_t const v = tileHist[t * 256u + uint32_t(tid)];
+                        before += t < blockIdx.x ? v : 0u;
+                        total += v;
+                    }
+                }
+                else
+                {
+                    before = tileHist[size_t(tid) * ntile + blockIdx.x];
+                    total = totals[tid];
+                }
+                uint32_t incl = total;
+#pragma unroll
+                for(int d = 1; d < 32; d <<= 1)
+                {
+                    uint32_t const o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if(lane >= d)
+                        incl += o;
+                }
+                if(lane == 31)
+                    warpCnt[0][warp] = incl;
+                __syncthreads();
+                uint32_t base = 0;
+                for(int w = 0; w < warp; ++w)
+                    base += warpCnt[0][w];
+                running[tid] = base + incl - total + before;
+                __syncthreads();
+            }
             uint32_t const lanesBelow = (1u << lane) - 1u;
-            uint32_t const base = blockIdx.x * uint32_t(kTile);
-            for(int r = 0; r < kRounds; ++r)
+            uint32_t const base = blockIdx.x * uint32_t(kThreads) * rounds;
+            for(uint32_t r = 0; r < rounds; ++r)
             {
                 for(int w = 0; w < kThreads / 32; ++w)
                     warpCnt[w][tid] = 0;
                 __syncthreads();
-                uint32_t const i = base + uint32_t(r) * kThreads + tid;
+                uint32_t const i = base + r * kThreads + uint32_t(tid);
                 bool const valid = i < n;
                 uint32_t key = 0, val = 0;
                 if(valid)
@@ -202,9 +306,7 @@ namespace sph
 
     size_t radixScratchWords(uint32_t n)
     {
-        uint32_t const ntile = (n + kTile - 1) / kTile;
-        size_t const hist = size_t(256) * ntile;
-        return 2 * hist + scanScratchWords(uint32_t(hist));
+        return size_t(256) * tileCount(n) + 256;
     }
 
     bool radixSortPairs(
@@ -220,21 +322,25 @@ namespace sph
         bool inB = false;
         if(n == 0)
             return inB;
-        uint32_t const ntile = (n + kTile - 1) / kTile;
-        size_t const hist = size_t(256) * ntile;
+        uint32_t const rounds = tileRounds(n), ntile = tileCount(n);
+        bool const few = ntile <= kFewTiles;
         uint32_t* tileHist = scratch;
-        uint32_t* tileOff = scratch + hist;
-        uint32_t* scanScr = scratch + 2 * hist;
+        uint32_t* totals = scratch + size_t(256) * ntile;
         for(int shift = 0; shift < bits; shift += 8)
         {
             uint32_t const* kin = inB ? keysB : keysA;
             uint32_t const* vin = inB ? valsB : valsA;
             uint32_t* kout = inB ? keysA : keysB;
             uint32_t* vout = inB ? valsA : valsB;
-            kRadixHist<<<ntile, kThreads, 0, s>>>(kin, n, shift, tileHist, ntile);
+            kRadixHist<<<ntile, kThreads, 0, s>>>(kin, n, shift, rounds, tileHist, ntile, few);
             countLaunches(1);
-            exclusiveScan(tileHist, tileOff, uint32_t(hist), scanScr, s);
-            kRadixScatter<<<ntile, kThreads, 0, s>>>(kin, vin, kout, vout, n, shift, tileOff, ntile);
+            if(!few)
+            {
+                kRadixRows<<<256, kThreads, 0, s>>>(tileHist, ntile, totals);
+                countLaunches(1);
+            }
+            kRadixScatter<<<ntile, kThreads, 0, s>>>(
+                kin, vin, kout, vout, n, shift, rounds, tileHist, totals, ntile, few);
             countLaunches(1);
             inB = !inB;
         }

@@ -148,7 +148,8 @@ namespace sph
         return D4{a.x, a.y, b.x, b.y};
     }
 
-    //! Cell index ranges in sorted order: [start, mid) targets, [mid, end) other sources.
+    //! Cell index ranges in sorted order: [start, mid) targets, [mid, end) other
+    //! sources.  The three arrays are one allocation (start, then mid, then end).
     struct Cells
     {
         uint32_t* start;
@@ -196,6 +197,9 @@ namespace sph
         unsigned long long* hmaxBits; //!< max h of the box's particles (ordered bits; the grid follows it)
         unsigned long long* hminBits; //!< min h of the box's particles (ordered bits; two levels when small enough)
     };
+
+    //! Start value of the per-box CFL minimum (ordered bits of a number above 1e300).
+    constexpr unsigned long long kNoDt = 0x7f7f7f7f7f7f7f7full;
 
     struct DevCtx
     {

@@ -17,6 +17,23 @@ namespace sph
     {
         constexpr int kThreads = 256;
 
+        //! Zeroes what the passes of this build add to (one block): a memset node
+        //! per word cost a small system's step more than its kernels.
+        __device__ __forceinline__ void clearStep(DevCtx const& c)
+        {
+            if(threadIdx.x == 0)
+            {
+                c.scal->pairs = 0;
+                c.scal->candidates = 0;
+                *c.work = 0;
+            }
+            for(uint32_t b = threadIdx.x; b < c.nbox; b += blockDim.x)
+            {
+                c.bs.chBits[b] = 0;
+                c.bs.dtBits[b] = kNoDt;
+            }
+        }
+
         //! Drift (Movable): x += v dt with periodic wrap; then the cell key.  The
         //! product and the sum are rounded separately, as the reference's CPU
         //! path evaluates PushVelocity (PushVelocity.hpp:38-41), so the FP64
@@ -26,6 +43,8 @@ namespace sph
         __global__ void __launch_bounds__(kThreads) kDriftKeys(DevCtx c, bool drift)
         {
             uint32_t const p = blockIdx.x * blockDim.x + threadIdx.x;
+            if(blockIdx.x == 0)
+                clearStep(c);
             if(p >= c.n)
                 return;
             uint8_t const role = c.cur.role[p];
@@ -160,6 +179,9 @@ namespace sph
             c.alt.box[p] = b;
             uint8_t const role = c.cur.role[q];
             c.alt.role[p] = role;
+            // no row until the neighbour build writes one
+            c.lists.count[p] = 0xffffffffu;
+            c.lists.rowLen[p] = 0;
             if(!isSource(role))
                 return;
             BoxDev const& B = c.boxes[b];
@@ -420,18 +442,18 @@ namespace sph
         }
 
         //! Largest and smallest h of each box's particles, as ordered bits.  A
-        //! warp walks kHmaxRun consecutive groups of 32 particles (each group one
+        //! warp walks `run` consecutive groups of 32 particles (each group one
         //! coalesced load) and keeps a running maximum and minimum while every
         //! particle of a group is in the warp's current box.  After the first
         //! neighbour build the particles are box-sorted, so one pair of atomics
         //! serves a whole run instead of every group: the boxes' 512 addresses
         //! otherwise serialise about 2 n / 32 atomics in L2.  A group that spans
         //! boxes falls back to per-particle atomics.
-        constexpr int kHmaxRun = 16;
-        __global__ void __launch_bounds__(kThreads) kBoxHmax(DevCtx c)
+        constexpr uint32_t kMaxHmaxRun = 16;
+        __global__ void __launch_bounds__(kThreads) kBoxHmax(DevCtx c, uint32_t run)
         {
             int const lane = threadIdx.x & 31;
-            uint32_t const base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32u * kHmaxRun);
+            uint32_t const base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32u * run);
             int cur = -1; // warp-uniform: the box the running extrema belong to
             double m = 0.0, mn = 1e300;
             auto flush = [&]()
@@ -453,9 +475,9 @@ namespace sph
                 m = 0.0;
                 mn = 1e300;
             };
-            for(int it = 0; it < kHmaxRun; ++it)
+            for(uint32_t it = 0; it < run; ++it)
             {
-                uint32_t const g = base + uint32_t(it) * 32u;
+                uint32_t const g = base + it * 32u;
                 if(g >= c.n)
                     break;
                 uint32_t const p = g + uint32_t(lane);
@@ -557,32 +579,56 @@ namespace sph
                 B.msub = B.levels == 2 ? msub : 1u;
                 B.e1 = e1;
                 B.nItems = B.levels == 2 ? B.ncells * (1u + msub) : B.ncells;
-                for(int sl = 0; sl < 32; ++sl)
-                {
-                    int const o[3] = {stencilOff(sl, 0), stencilOff(sl, 1), stencilOff(sl, 2)};
-                    bool const used = sl < 27;
-                    c.shift32[size_t(b) * 32 + sl] = used ? make_float4(
-                                                                float(o[0]) * B.edgef[0],
-                                                                float(o[1]) * B.edgef[1],
-                                                                float(o[2]) * B.edgef[2],
-                                                                0.f)
-                                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-                    c.shift64[size_t(b) * 32 + sl] = used ? D4{double(o[0]) * B.edge[0], double(o[1]) * B.edge[1],
-                                                                double(o[2]) * B.edge[2], 0.0}
-                                                          : D4{0.0, 0.0, 0.0, 0.0};
-                }
+                // for the next build's extrema
+                c.bs.hmaxBits[b] = 0;
+                c.bs.hminBits[b] = ~0ull;
             }
             __syncthreads();
-            if(threadIdx.x == 0)
+            // stencil shift tables, one entry per thread
+            for(uint32_t i = threadIdx.x; i < c.nbox * 32u; i += blockDim.x)
             {
-                uint32_t base = 0;
-                for(uint32_t b = 0; b < c.nbox; ++b)
-                {
-                    c.boxes[b].activeBase = base;
-                    base += c.boxes[b].nItems;
-                }
-                *c.activeTotal = base;
+                BoxDev const& B = c.boxes[i >> 5];
+                int const sl = int(i & 31u);
+                bool const used = sl < 27;
+                int const o[3] = {stencilOff(sl, 0), stencilOff(sl, 1), stencilOff(sl, 2)};
+                c.shift32[i] = used ? make_float4(
+                                          float(o[0]) * B.edgef[0], float(o[1]) * B.edgef[1], float(o[2]) * B.edgef[2], 0.f)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                c.shift64[i] = used ? D4{double(o[0]) * B.edge[0], double(o[1]) * B.edge[1], double(o[2]) * B.edge[2], 0.0}
+                                    : D4{0.0, 0.0, 0.0, 0.0};
             }
+            // prefix of the boxes' work items
+            __shared__ uint32_t warpTot[32];
+            int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = int(blockDim.x) / 32;
+            uint32_t base = 0;
+            for(uint32_t b0 = 0; b0 < c.nbox; b0 += blockDim.x)
+            {
+                uint32_t const b = b0 + threadIdx.x;
+                uint32_t const v = b < c.nbox ? c.boxes[b].nItems : 0u;
+                uint32_t incl = v;
+#pragma unroll
+                for(int d = 1; d < 32; d <<= 1)
+                {
+                    uint32_t const o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if(lane >= d)
+                        incl += o;
+                }
+                if(lane == 31)
+                    warpTot[warp] = incl;
+                __syncthreads();
+                uint32_t before = base;
+                for(int w = 0; w < warps; ++w)
+                {
+                    if(w < warp)
+                        before += warpTot[w];
+                    base += warpTot[w];
+                }
+                if(b < c.nbox)
+                    c.boxes[b].activeBase = before + incl - v;
+                __syncthreads();
+            }
+            if(threadIdx.x == 0)
+                *c.activeTotal = base;
         }
 
         //! Level-1 block range of each level-0 cell of a two-level box: the union
@@ -767,9 +813,8 @@ namespace sph
 
     void launchCellRanges(DevCtx const& c, uint32_t const* sortedKeys, cudaStream_t s)
     {
-        cudaMemsetAsync(c.cells.start, 0, size_t(c.cells.ncells) * 4, s);
-        cudaMemsetAsync(c.cells.mid, 0, size_t(c.cells.ncells) * 4, s);
-        cudaMemsetAsync(c.cells.end, 0, size_t(c.cells.ncells) * 4, s);
+        // start, mid and end are one array
+        cudaMemsetAsync(c.cells.start, 0, size_t(c.cells.ncells) * 12, s);
         if(c.n)
         {
             kCellRanges<<<(c.n + kThreads - 1) / kThreads, kThreads, 0, s>>>(sortedKeys, c.n, c.cells);
@@ -895,12 +940,13 @@ namespace sph
 
     void launchGridUpdate(DevCtx const& c, int support, cudaStream_t s)
     {
-        cudaMemsetAsync(c.bs.hmaxBits, 0, sizeof(unsigned long long) * c.nbox, s);
-        cudaMemsetAsync(c.bs.hminBits, 0xff, sizeof(unsigned long long) * c.nbox, s);
         if(c.n)
         {
-            uint32_t const perBlock = uint32_t(kThreads / 32) * 32u * uint32_t(kHmaxRun);
-            kBoxHmax<<<(c.n + perBlock - 1) / perBlock, kThreads, 0, s>>>(c);
+            // runs of 16 groups once they fill 16 warps per SM, shorter ones before
+            uint32_t const fill = c.n / (32u * 148u * 16u);
+            uint32_t const run = fill < 1u ? 1u : (fill > kMaxHmaxRun ? kMaxHmaxRun : fill);
+            uint32_t const perBlock = uint32_t(kThreads) * run;
+            kBoxHmax<<<(c.n + perBlock - 1) / perBlock, kThreads, 0, s>>>(c, run);
             countLaunches(1);
         }
         kGrid<<<1, 256, 0, s>>>(c, support);
