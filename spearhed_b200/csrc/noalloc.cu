@@ -35,7 +35,7 @@
 // Those inputs are found by the same launch sequence that computes rho, so
 // on either return rho holds values that must not be used.  Every call waits
 // for its own work on `stream` before it returns.
-#include "sph_launch.hpp"
+#include "pair_common.cuh"
 
 #include <cmath>
 #include <cstdio>
@@ -104,7 +104,7 @@ namespace
     //! periodic ones included), status[1] non-finite positions and masses or
     //! smoothing lengths that are not finite and positive.
     __global__ void kKeysInput(
-        sph::BoxDev const* __restrict__ box,
+        sph::BoxDev const B,
         uint32_t n,
         double const* __restrict__ x,
         double const* __restrict__ y,
@@ -118,7 +118,6 @@ namespace
         uint32_t const p = blockIdx.x * blockDim.x + threadIdx.x;
         if(p >= n)
             return;
-        sph::BoxDev const& B = *box;
         double const pos[3] = {x[p], y[p], z[p]};
         double const mp = m[p], hp = h[p];
         bool nonfinite = !(isfinite(mp) && mp > 0.0) || !(isfinite(hp) && hp > 0.0);
@@ -141,7 +140,7 @@ namespace
 
     template<typename V4, typename T>
     __global__ void kPackSorted(
-        sph::BoxDev const* __restrict__ box,
+        sph::BoxDev const B,
         uint32_t n,
         uint32_t const* __restrict__ perm,
         double const* __restrict__ x,
@@ -156,7 +155,6 @@ namespace
         if(p >= n)
             return;
         uint32_t const q = perm[p];
-        sph::BoxDev const& B = *box;
         double const pos[3] = {x[q], y[q], z[q]};
         double rel[3];
         for(int a = 0; a < 3; ++a)
@@ -168,143 +166,196 @@ namespace
         hc[p] = T(h[q]);
     }
 
-    __device__ __forceinline__ float mulRn(float a, float b)
-    {
-        return __fmul_rn(a, b);
-    }
-    __device__ __forceinline__ float addRn(float a, float b)
-    {
-        return __fadd_rn(a, b);
-    }
-    __device__ __forceinline__ double mulRn(double a, double b)
-    {
-        return __dmul_rn(a, b);
-    }
-    __device__ __forceinline__ double addRn(double a, double b)
-    {
-        return __dadd_rn(a, b);
-    }
+    //! Density with the accumulation inside the cull (no neighbour list): a warp
+    //! takes a group of up to kGroup targets of one cell (few particles: smaller
+    //! groups, so that more warps share a cell), stages the candidates of the
+    //! 27-cell stencil that come within the cull radius of the group's bounding
+    //! box into shared memory, shift applied, and each target sums them with
+    //! 32 / kGroup or more lanes.  Every staged candidate is evaluated: about one
+    //! in three is accepted, and a divergent walk over the accepted ones would cost
+    //! more than the rejected evaluations.  A thread per target reading the
+    //! stencil from global memory waited for one dependent 16-byte load per
+    //! candidate with a third of its lanes.  Whole calls, 40 neighbours each, thread
+    //! per target -> staged: 250 k FP32 cubic 490 -> 222 us, FP64 625 -> 304; 6 k
+    //! FP32 150 -> 67, FP64 168 -> 73 (the cell sort's share of that included).
+    //!
+    //! The acceptance rule is the list-based path's (unfused r^2 in x, y, z order
+    //! against R^2); the target itself is its candidate at r = 0, which gives the
+    //! self term.  FP32 lanes fold blocks of 8 candidates by TwoSum; lane sums are
+    //! added in FP64.  rho is written in input order.
+    constexpr int kWindow = 128; //!< staged candidates per warp
 
     template<typename T>
-    __device__ __forceinline__ T edgeT(sph::BoxDev const& B, int a);
-    template<>
-    __device__ __forceinline__ float edgeT<float>(sph::BoxDev const& B, int a)
+    __device__ __forceinline__ T boxDistance(T lo, T hi, T negX)
     {
-        return B.edgef[a];
-    }
-    template<>
-    __device__ __forceinline__ double edgeT<double>(sph::BoxDev const& B, int a)
-    {
-        return B.edge[a];
+        return fmax(fmax(sph::addRn(lo, negX), -sph::addRn(hi, negX)), T(0));
     }
 
-    //! Density with the accumulation inside the cull (no neighbour list):
-    //! one warp per cell, each lane one target, candidates read straight from
-    //! the sorted records.  Same acceptance rule and summation order as the
-    //! list-based kernel; the FP32 variant folds blocks of 8 accepted terms
-    //! into a TwoSum-compensated sum.  rho is written in input order.
+    //! r from r^2: correctly rounded in FP32 (this path has no later pass to match).
+    __device__ __forceinline__ float distance(float r2)
+    {
+        return __fsqrt_rn(r2);
+    }
+    __device__ __forceinline__ double distance(double r2)
+    {
+        return r2 * sph::invDistance(r2);
+    }
+
     template<int K, typename V4, typename T>
-    __global__ void __launch_bounds__(kWarps * 32) kDensityInline(
-        sph::BoxDev const* __restrict__ box,
+    __global__ void __launch_bounds__(kWarps * 32) kDensityStaged(
+        sph::BoxDev const box,
         sph::Cells cells,
         uint32_t const* __restrict__ perm,
         V4 const* __restrict__ pm,
         T const* __restrict__ hc,
-        double h0,
+        T R2g,
+        uint32_t group,
+        int partShift,
         double* __restrict__ rhoOut)
     {
-        sph::BoxDev const& B = *box;
+        __shared__ V4 staged[kWarps][kWindow];
         int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        T const sup = T(sph::Kern<K>::support);
-        T const Rg = mulRn(sup, T(h0));
-        T const R2g = mulRn(Rg, Rg);
-        for(uint32_t cell = blockIdx.x * kWarps + warp; cell < cells.ncells; cell += gridDim.x * kWarps)
+        V4* const win = staged[warp];
+        uint32_t const items = cells.ncells << partShift;
+        for(uint32_t q = blockIdx.x * kWarps + uint32_t(warp); q < items; q += gridDim.x * kWarps)
         {
-            uint32_t const tBeg = cells.start[cell], tEnd = cells.mid[cell];
+            uint32_t const cell = q >> partShift;
+            uint32_t const tBeg = cells.start[cell] + (q & ((1u << partShift) - 1u)) * group, tEnd = cells.mid[cell];
             if(tBeg >= tEnd)
                 continue;
-            int const cc[3] = {int(cell % uint32_t(B.n[0])), int((cell / uint32_t(B.n[0])) % uint32_t(B.n[1])),
-                               int(cell / (uint32_t(B.n[0]) * uint32_t(B.n[1])))};
-            for(uint32_t tc = tBeg; tc < tEnd; tc += 32)
+            // lane d < 27: the source range and image shift of stencil slot d
+            uint32_t sBeg = 0, cnt = 0;
+            T sh[3] = {T(0), T(0), T(0)};
+            if(lane < 27)
             {
-                uint32_t const t = tc + uint32_t(lane);
-                if(t >= tEnd)
-                    continue;
-                V4 const own = sph::ld4(pm + t);
-                T const hi = hc[t];
+                uint32_t const n0 = uint32_t(box.n[0]), n1 = uint32_t(box.n[1]);
+                int const cc[3] = {int(cell % n0), int((cell / n0) % n1), int(cell / (n0 * n1))};
+                int nc[3];
+                bool ok = true;
+#pragma unroll
+                for(int a = 0; a < 3; ++a)
+                {
+                    int const o = sph::stencilOff(lane, a);
+                    nc[a] = cc[a] + o;
+                    if(nc[a] < 0 || nc[a] >= box.n[a])
+                    {
+                        if(box.periodic[a])
+                            nc[a] = (nc[a] + box.n[a]) % box.n[a];
+                        else
+                            ok = false;
+                    }
+                    sh[a] = T(o) * sph::edgeOf<T>(box, a);
+                }
+                if(ok)
+                {
+                    uint32_t const ncell = (uint32_t(nc[2]) * n1 + uint32_t(nc[1])) * n0 + uint32_t(nc[0]);
+                    sBeg = cells.start[ncell];
+                    cnt = cells.end[ncell] - sBeg;
+                }
+            }
+            uint32_t pre = cnt;
+#pragma unroll
+            for(int d = 1; d < 32; d <<= 1)
+            {
+                uint32_t const o = __shfl_up_sync(0xffffffffu, pre, d);
+                if(lane >= d)
+                    pre += o;
+            }
+            uint32_t const total = __shfl_sync(0xffffffffu, pre, 31);
+            pre -= cnt;
+            for(uint32_t tc = tBeg; tc < tEnd; tc += group << partShift)
+            {
+                uint32_t const nt = min(group, tEnd - tc);
+                int S = 1; // lanes per target
+                while(nt * uint32_t(2 * S) <= 32u)
+                    S *= 2;
+                uint32_t const t = tc + uint32_t(lane) / uint32_t(S);
+                int const sub = lane & (S - 1);
+                bool const act = t < tc + nt;
+                V4 own{};
+                T hi = T(1);
+                if(act)
+                {
+                    own = sph::ld4(pm + t);
+                    hi = hc[t];
+                }
+                T bLo[3], bHi[3];
+                T const x[3] = {own.x, own.y, own.z};
+#pragma unroll
+                for(int a = 0; a < 3; ++a)
+                {
+                    bLo[a] = sph::warpMinT<T>(act ? x[a] : T(1e30f));
+                    bHi[a] = sph::warpMaxT<T>(act ? x[a] : T(-1e30f));
+                }
+                // rounding is monotone, so with the radius widened by 2^-10 the box
+                // test passes every candidate that the exact test accepts
+                T const reach = R2g * (T(1) + T(1.0 / 1024.0));
                 sph::HConst<T> const hk = sph::hconst<K, T>(hi);
-                T acc = own.w * sph::kernelW<K, T>(T(0), hk);
-                sph::CompAcc comp;
-                T part = T(0);
-                int inBlock = 0;
-                for(int sl = 0; sl < 27; ++sl)
+                sph::Acc<T> rho;
+                uint32_t next = 0; // stencil position to stage
+                while(next < total)
                 {
-                    int nc[3];
-                    bool ok = true;
-                    T sh[3];
-                    for(int a = 0; a < 3; ++a)
+                    uint32_t m = 0;
+                    __syncwarp();
+                    while(next < total && m + 32u <= uint32_t(kWindow))
                     {
-                        int const o = sph::stencilOff(sl, a);
-                        nc[a] = cc[a] + o;
-                        if(nc[a] < 0 || nc[a] >= B.n[a])
+                        uint32_t const p = next + uint32_t(lane);
+                        // the last slot whose prefix is <= p
+                        int d = 0;
+#pragma unroll
+                        for(int step = 16; step >= 1; step >>= 1)
+                            if(__shfl_sync(0xffffffffu, pre, d + step) <= p)
+                                d += step;
+                        uint32_t const j = __shfl_sync(0xffffffffu, sBeg, d) + p - __shfl_sync(0xffffffffu, pre, d);
+                        T const sx = __shfl_sync(0xffffffffu, sh[0], d), sy = __shfl_sync(0xffffffffu, sh[1], d),
+                                sz = __shfl_sync(0xffffffffu, sh[2], d);
+                        bool pass = false;
+                        V4 c{};
+                        if(p < total)
                         {
-                            if(B.periodic[a])
-                                nc[a] = (nc[a] + B.n[a]) % B.n[a];
-                            else
-                                ok = false;
+                            c = sph::ld4(pm + j);
+                            c.x = -sph::addRn(c.x, sx);
+                            c.y = -sph::addRn(c.y, sy);
+                            c.z = -sph::addRn(c.z, sz);
+                            T const dx = boxDistance(bLo[0], bHi[0], c.x), dy = boxDistance(bLo[1], bHi[1], c.y),
+                                    dz = boxDistance(bLo[2], bHi[2], c.z);
+                            pass = dx * dx + dy * dy + dz * dz < reach;
                         }
-                        sh[a] = T(o) * edgeT<T>(B, a);
+                        uint32_t const passed = __ballot_sync(0xffffffffu, pass);
+                        if(pass)
+                            win[m + uint32_t(__popc(passed & ((1u << lane) - 1u)))] = c;
+                        m += uint32_t(__popc(passed));
+                        next += 32;
                     }
-                    if(!ok)
-                        continue;
-                    uint32_t const ncell = (uint32_t(nc[2]) * uint32_t(B.n[1]) + uint32_t(nc[1])) * uint32_t(B.n[0])
-                                           + uint32_t(nc[0]);
-                    uint32_t const s = cells.start[ncell], e = cells.end[ncell];
-                    for(uint32_t j = s; j < e; ++j)
+                    __syncwarp();
+                    uint32_t k = uint32_t(sub);
+                    while(k < m)
                     {
-                        if(sl == sph::kCentreSlot && j == t)
-                            continue;
-                        V4 const pj = sph::ld4(pm + j);
-                        T const qx = pj.x + sh[0], qy = pj.y + sh[1], qz = pj.z + sh[2];
-                        T const dx = own.x - qx, dy = own.y - qy, dz = own.z - qz;
-                        // unfused, x then y then z: the acceptance test of the list-based kernel
-                        T const r2 = addRn(addRn(mulRn(dx, dx), mulRn(dy, dy)), mulRn(dz, dz));
-                        if(r2 < R2g)
+                        for(int b = 0; b < sph::kBlock && k < m; ++b, k += uint32_t(S))
                         {
-                            T const r = r2 > T(0) ? r2 * (T(1) / sqrt(r2)) : T(0);
-                            T const term = pj.w * sph::kernelW<K, T>(r, hk);
-                            if constexpr(sizeof(T) == 4)
-                            {
-                                part += term;
-                                if(++inBlock == 8)
-                                {
-                                    comp.fold(float(part));
-                                    part = T(0);
-                                    inBlock = 0;
-                                }
-                            }
-                            else
-                                acc += term;
+                            V4 const c = win[k];
+                            T const dx = sph::addRn(own.x, c.x), dy = sph::addRn(own.y, c.y), dz = sph::addRn(own.z, c.z);
+                            T const r2 = sph::addRn(
+                                sph::addRn(sph::mulRn(dx, dx), sph::mulRn(dy, dy)), sph::mulRn(dz, dz));
+                            T const w = c.w * sph::kernelW<K, T>(distance(r2), hk);
+                            rho.add(r2 < R2g ? w : T(0));
                         }
+                        rho.fold();
                     }
                 }
-                double value;
-                if constexpr(sizeof(T) == 4)
-                {
-                    comp.fold(float(part));
-                    comp.fold(float(acc));
-                    value = comp.value();
-                }
-                else
-                    value = double(acc);
-                rhoOut[perm[t]] = value;
+                double v = rho.value();
+                for(int o = 1; o < S; o <<= 1)
+                    v += __shfl_xor_sync(0xffffffffu, v, o);
+                if(act && sub == 0)
+                    rhoOut[perm[t]] = v;
             }
         }
     }
 
     template<int K, typename V4, typename T>
-    void launchInline(
-        sph::BoxDev const* box,
+    void launchStaged(
+        sph::BoxDev const& box,
+        uint32_t n,
         sph::Cells const& cells,
         uint32_t const* perm,
         V4 const* pm,
@@ -313,16 +364,28 @@ namespace
         double* rho,
         cudaStream_t s)
     {
-        uint32_t blocks = (cells.ncells + kWarps - 1) / kWarps;
+        // Targets per warp: a cell's, at most 32, halved while the groups would
+        // not give each of 16 warps per SM one.
+        uint32_t group = 32;
+        int partShift = 0;
+        while(group > 4 && uint64_t(n) < uint64_t(group) * 148u * 16u)
+        {
+            group /= 2;
+            ++partShift;
+        }
+        uint32_t blocks = ((cells.ncells << partShift) + kWarps - 1) / kWarps;
         blocks = blocks > 148u * 32u ? 148u * 32u : blocks;
         // the global cull radius only: pair-max calls are refused before any launch
-        kDensityInline<K, V4, T><<<blocks, kWarps * 32, 0, s>>>(box, cells, perm, pm, hc, p.h0, rho);
+        T const Rg = T(sph::Kern<K>::support) * T(p.h0);
+        kDensityStaged<K, V4, T>
+            <<<blocks, kWarps * 32, 0, s>>>(box, cells, perm, pm, hc, T(Rg * Rg), group, partShift, rho);
         sph::countLaunches(1);
     }
 
     template<typename V4, typename T>
-    void launchInlineK(
-        sph::BoxDev const* box,
+    void launchStagedK(
+        sph::BoxDev const& box,
+        uint32_t n,
         sph::Cells const& cells,
         uint32_t const* perm,
         V4 const* pm,
@@ -332,11 +395,11 @@ namespace
         cudaStream_t s)
     {
         if(p.kernel == SPH_KERNEL_QUINTIC)
-            launchInline<SPH_KERNEL_QUINTIC>(box, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_QUINTIC>(box, n, cells, perm, pm, hc, p, rho, s);
         else if(p.kernel == SPH_KERNEL_WENDLAND_C2)
-            launchInline<SPH_KERNEL_WENDLAND_C2>(box, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_WENDLAND_C2>(box, n, cells, perm, pm, hc, p, rho, s);
         else
-            launchInline<SPH_KERNEL_CUBIC>(box, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_CUBIC>(box, n, cells, perm, pm, hc, p, rho, s);
     }
 } // namespace
 
@@ -411,7 +474,6 @@ int sph_density_noalloc(
     uint32_t const nn = uint32_t(n);
     bool const fp64 = p.precision == SPH_PREC_FP64;
     Carve cv{static_cast<unsigned char*>(base)};
-    sph::BoxDev* dBox = cv.take<sph::BoxDev>(1);
     uint32_t* status = cv.take<uint32_t>(4);
     uint32_t* keysA = cv.take<uint32_t>(nn);
     uint32_t* valsA = cv.take<uint32_t>(nn);
@@ -448,8 +510,7 @@ int sph_density_noalloc(
     (void)cudaGetLastError();
     // Everything below is stream-ordered; nothing that must start at zero is
     // assumed to be zero from an earlier call.
-    if(cudaMemcpyAsync(dBox, &bd, sizeof(bd), cudaMemcpyHostToDevice, s) != cudaSuccess
-       || cudaMemsetAsync(status, 0, 4 * sizeof(uint32_t), s) != cudaSuccess)
+    if(cudaMemsetAsync(status, 0, 4 * sizeof(uint32_t), s) != cudaSuccess)
         return failNoAlloc(SPH_ERR_CUDA, "sph_density_noalloc: stream operation failed");
     auto launched = [](char const* what) -> int
     {
@@ -460,7 +521,7 @@ int sph_density_noalloc(
         return failNoAlloc(SPH_ERR_CUDA, std::string("sph_density_noalloc: ") + what + ": " + cudaGetErrorString(e));
     };
     unsigned const g = (nn + kThreads - 1) / kThreads;
-    kKeysInput<<<g, kThreads, 0, s>>>(dBox, nn, x, y, z, mass, h, keysA, valsA, status);
+    kKeysInput<<<g, kThreads, 0, s>>>(bd, nn, x, y, z, mass, h, keysA, valsA, status);
     sph::countLaunches(1);
     if((st = launched("cell keys")))
         return st;
@@ -480,19 +541,19 @@ int sph_density_noalloc(
         return st;
     if(fp64)
     {
-        kPackSorted<sph::D4, double><<<g, kThreads, 0, s>>>(dBox, nn, perm, x, y, z, mass, h, pm64, hc64);
+        kPackSorted<sph::D4, double><<<g, kThreads, 0, s>>>(bd, nn, perm, x, y, z, mass, h, pm64, hc64);
         sph::countLaunches(1);
         if((st = launched("packing")))
             return st;
-        launchInlineK<sph::D4, double>(dBox, cells, perm, pm64, hc64, p, rho, s);
+        launchStagedK<sph::D4, double>(bd, nn, cells, perm, pm64, hc64, p, rho, s);
     }
     else
     {
-        kPackSorted<float4, float><<<g, kThreads, 0, s>>>(dBox, nn, perm, x, y, z, mass, h, pm32, hc32);
+        kPackSorted<float4, float><<<g, kThreads, 0, s>>>(bd, nn, perm, x, y, z, mass, h, pm32, hc32);
         sph::countLaunches(1);
         if((st = launched("packing")))
             return st;
-        launchInlineK<float4, float>(dBox, cells, perm, pm32, hc32, p, rho, s);
+        launchStagedK<float4, float>(bd, nn, cells, perm, pm32, hc32, p, rho, s);
     }
     if((st = launched("density")))
         return st;
