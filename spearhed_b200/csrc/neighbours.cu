@@ -422,6 +422,13 @@ namespace sph
                 // or, for a level-0 target, the level-1 block (all sub-cells) of each
                 // of those 27 cells.  Each carries its source range and the level-0
                 // stencil slot of its image.
+                //
+                // Order: a periodic axis of one or two cells shows the same cell through
+                // two or three images.  Such axes run fastest, equal cells adjacent (-1,
+                // +1, 0), so a row lists a cell's images one after another and the lanes
+                // of a pair pass, which stand at different images, stay on the same
+                // lines of records: 16.8 -> 12 lines a request on the Orszag-Tang slab
+                // (one cell thick), force pass 0.643 -> 0.600 ms.
                 int const nDesc = 27 + (B.levels == 2 ? 27 : 0);
                 auto describe = [&](int d, uint32_t& sBeg, uint32_t& sCnt, uint32_t& slot, T sh[3])
                 {
@@ -436,6 +443,22 @@ namespace sph
                     bool const fine = d >= 27;
                     int const k = fine ? d - 27 : d;
                     bool const fineCell = fine && lt; // a level-1 neighbour of a level-1 target
+                    bool thin[3];
+                    int nThin = 0, before = 0, off[3];
+#pragma unroll
+                    for(int a = 0; a < 3; ++a)
+                    {
+                        thin[a] = B.periodic[a] && (fineCell ? B.n[a] << (B.m[a] - 1) : B.n[a]) <= 2;
+                        nThin += thin[a] ? 1 : 0;
+                    }
+#pragma unroll
+                    for(int a = 0; a < 3; ++a)
+                    {
+                        int const place = thin[a] ? before : nThin + a - before;
+                        before += thin[a] ? 1 : 0;
+                        int const digit = stencilOff(k, place) + 1;
+                        off[a] = !thin[a] ? digit - 1 : (digit == 2 ? 0 : 2 * digit - 1);
+                    }
 #pragma unroll
                     for(int a = 0; a < 3; ++a)
                     {
@@ -445,14 +468,14 @@ namespace sph
                             // fine-grid neighbour; its level-0 parent (image-aware) gives o
                             int const sh = B.m[a] - 1; // splits are 1 or 2
                             int const n1 = n0 << sh;
-                            int const fa = ct[a] + stencilOff(k, a);
+                            int const fa = ct[a] + off[a];
                             o[a] = (fa >> sh) - c0[a];
                             f[a] = fa < 0 || fa >= n1 ? (B.periodic[a] ? (fa + n1) % n1 : -1) : fa;
                             ok = ok && f[a] >= 0;
                         }
                         else
                         {
-                            o[a] = stencilOff(k, a);
+                            o[a] = off[a];
                             int ca = c0[a] + o[a];
                             if(ca < 0 || ca >= n0)
                             {
