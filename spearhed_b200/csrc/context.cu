@@ -815,7 +815,7 @@ int sph_ctx::growLists(uint32_t need, bool bestEffort)
     {
         // headroom only: the new rows are allocated beside the old ones, and a
         // context that cannot have them keeps the lists it has
-        if(alloc(list, size_t(n) * capN + sph::kRowSlack) != SPH_OK)
+        if(alloc(list, sph::listWords(n, capN)) != SPH_OK)
         {
             cudaGetLastError();
             return SPH_OK;
@@ -833,7 +833,7 @@ int sph_ctx::growLists(uint32_t need, bool bestEffort)
     }
     if(!list)
     {
-        int const st = alloc(list, size_t(n) * capN + sph::kRowSlack);
+        int const st = alloc(list, sph::listWords(n, capN));
         if(st)
             return st;
     }

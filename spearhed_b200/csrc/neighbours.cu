@@ -191,18 +191,54 @@ namespace sph
             ch.nR2 = -mulRn(Ri, Ri);
         }
 
+        //! One target's share of a slab during the write-out: x its mask, bit l for
+        //! lane l's candidate; then, FP32 (interleaved rows): y one before the slab's
+        //! first place in the row, z the row's start; FP64: y the two added up.
+        template<typename T>
+        struct RowRef;
+        template<>
+        struct RowRef<float>
+        {
+            using Type = uint4;
+            static __device__ __forceinline__ uint4 make(uint32_t bits, uint32_t row, uint32_t k)
+            {
+                return make_uint4(bits, k - 1u, row, 0u);
+            }
+            static __device__ __forceinline__ uint32_t place(uint4 r, uint32_t below)
+            {
+                return r.z + rowPlace<float>(r.y + below);
+            }
+        };
+        template<>
+        struct RowRef<double>
+        {
+            using Type = uint2;
+            static __device__ __forceinline__ uint2 make(uint32_t bits, uint32_t row, uint32_t k)
+            {
+                return make_uint2(bits, row + k - 1u);
+            }
+            static __device__ __forceinline__ uint32_t place(uint2 r, uint32_t below)
+            {
+                return r.y + below;
+            }
+        };
+
         //! Stores a candidate's entry into one target's row when the target
-        //! accepts it.  r.x: the target's mask, bit l for lane l's candidate; r.y:
-        //! one before the slab's first row position; up = 31 - lane.  The bits up
-        //! to the lane's own are moved to the top: the sign is its own bit, the
-        //! population its place.  The store is predicated (a branch around it
-        //! would add the warp's divergence bookkeeping to every target).
-        __device__ __forceinline__ void storeEntry(uint2 r, uint32_t up, uint32_t* rows, uint32_t ent)
+        //! accepts it; up = 31 - lane.  The mask's bits up to the lane's own are
+        //! moved to the top: the sign is its own bit, the population its place.
+        //! The store is predicated (a branch around it would add the warp's
+        //! divergence bookkeeping to every target).
+        template<typename T>
+        __device__ __forceinline__ void storeEntry(
+            typename RowRef<T>::Type r,
+            uint32_t up,
+            uint32_t* rows,
+            uint32_t ent)
         {
             uint32_t const b = r.x << up;
             asm volatile("{ .reg .pred q; setp.lt.s32 q, %0, 0; @q st.global.u32 [%1], %2; }"
                          :
-                         : "r"(b), "l"(rows + (r.y + uint32_t(__popc(b)))), "r"(ent)
+                         : "r"(b), "l"(rows + RowRef<T>::place(r, uint32_t(__popc(b)))), "r"(ent)
                          : "memory");
         }
 
@@ -231,7 +267,7 @@ namespace sph
             T const* sH,
             uint32_t const* sEnt,
             uint32_t const* sSelf,
-            uint2* sRow,
+            typename RowRef<T>::Type* sRow,
             uint32_t tc,
             uint32_t nt,
             uint32_t m,
@@ -245,7 +281,7 @@ namespace sph
             int const S = ch.S;
             uint32_t const selfq = ch.act ? sSelf[ch.t - tc] : ~0u;
             uint32_t const nSlab = (m + 31u) >> 5;
-            uint32_t const rowOff = (ch.t - tc) * cap;
+            uint32_t const rowOff = rowStart<T>(ch.t, cap) - rowStart<T>(tc & ~3u, cap);
             uint32_t const up = 31u - uint32_t(lane);
             for(uint32_t g0 = 0; g0 < nSlab; g0 += uint32_t(S))
             {
@@ -282,7 +318,7 @@ namespace sph
                     for(uint32_t over = min(cnt, k + cnt - cap); over > 0; --over)
                         mask &= mask - 1u;
                 __syncwarp();
-                sRow[lane] = make_uint2(__brev(mask), rowOff + k - 1u);
+                sRow[lane] = RowRef<T>::make(__brev(mask), rowOff, k);
                 __syncwarp();
                 if(S == 1)
                 {
@@ -292,7 +328,7 @@ namespace sph
                     for(uint32_t i = 0; i < nt; i += 8)
 #pragma unroll
                         for(uint32_t u = 0; u < 8; ++u)
-                            storeEntry(sRow[i + u], up, rows, ent);
+                            storeEntry<T>(sRow[i + u], up, rows, ent);
                     continue;
                 }
                 int const nS = int(min(uint32_t(S), nSlab - g0));
@@ -301,7 +337,7 @@ namespace sph
                     uint32_t const ent = sEnt[((g0 + uint32_t(s)) << 5) + uint32_t(lane)];
 #pragma unroll 4
                     for(uint32_t i = 0; i < nt; ++i)
-                        storeEntry(sRow[i * uint32_t(S) + uint32_t(s)], up, rows, ent);
+                        storeEntry<T>(sRow[i * uint32_t(S) + uint32_t(s)], up, rows, ent);
                 }
             }
         }
@@ -355,7 +391,8 @@ namespace sph
             uint32_t* const sSelf = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(smem) + kCols * kWarps * kCol)
                                     + kWarps * CAP + warp * 64;
             // per warp: each lane's slab mask and row position during the write-out
-            uint2* const sRow = reinterpret_cast<uint2*>(sSelf - warp * 64 + kWarps * 64) + warp * 32;
+            using Row = typename RowRef<T>::Type;
+            Row* const sRow = reinterpret_cast<Row*>(sSelf - warp * 64 + kWarps * 64) + warp * 32;
             Records<V4, T> const rec = records<T>(c);
             T const supT = T(c.support);
             T const Rg = mulRn(supT, T(h0));
@@ -721,7 +758,7 @@ namespace sph
                             uint32_t const first = tc + 32u * uint32_t(w);
                             cullChunk<T, PAIRMAX, CU>(
                                 ch, sNX, sNY, sNZ, sH, sEnt, sSelf + 32 * w, sRow, first, w ? ntB : ntA, m, supT, R2g,
-                                c.lists.list + size_t(first) * cap, cap, lane, countOnly);
+                                c.lists.list + rowStart<T>(size_t(first & ~3u), size_t(cap)), cap, lane, countOnly);
                             if(w)
                                 Bc = ch;
                             else
@@ -765,7 +802,7 @@ namespace sph
         constexpr size_t neighbourSmem()
         {
             return size_t(kWarps)
-                   * (colLen<CAP>() * (PM ? 4 : 3) * sizeof(T) + (CAP + 64) * sizeof(uint32_t) + 32 * sizeof(uint2));
+                   * (colLen<CAP>() * (PM ? 4 : 3) * sizeof(T) + (CAP + 64) * sizeof(uint32_t) + 32 * sizeof(typename RowRef<T>::Type));
         }
 
         // ---- launch-shape variants -------------------------------------------

@@ -51,7 +51,7 @@ namespace sph
         //! load 4 S entries as one 16-byte word each and exchange them (a 4-byte
         //! load per entry would cost a wavefront per target and entry).  `any` is
         //! a valid entry, fetched past the row's end.
-        template<int S, typename F, typename M, typename D>
+        template<typename T, int S, typename F, typename M, typename D>
         __device__ __forceinline__ void walkRow(
             uint32_t const* row,
             uint32_t n,
@@ -64,8 +64,9 @@ namespace sph
             if(n == 0)
                 return;
             uint32_t const lanes = ((1u << S) - 1u) << (threadIdx.x & (32u - S));
-            uint4 const* const row4 = reinterpret_cast<uint4 const*>(row) + sub;
-            uint4 e = spread<S>(row4[0], sub, lanes);
+            auto quad = [&](uint32_t k) // entries k .. k + 3, k a multiple of 4
+            { return *reinterpret_cast<uint4 const*>(row + rowPlace<T>(k)); };
+            uint4 e = spread<S>(quad(4 * sub), sub, lanes);
             fetch(sub < n ? e.x : any);
             for(uint32_t k = sub;; k += 4 * S)
             {
@@ -73,7 +74,7 @@ namespace sph
                 bool const more = k - sub + 4 * S < n;
                 uint4 next = e;
                 if(more)
-                    next = row4[(k - sub) / 4 + S];
+                    next = quad(k - sub + 4 * (S + sub));
                 if(k >= n)
                     break;
                 term(k + S < n ? e.y : any);
@@ -184,8 +185,8 @@ namespace sph
                     rho.add(pj.w * kernelW<K, T>(r2 * invDistance(r2), hk));
                 };
                 uint32_t const n = min(c.lists.rowLen[t], c.lists.cap);
-                walkRow<S>(
-                    c.lists.list + size_t(t) * c.lists.cap, n, sub, packEntry(t, kCentreSlot), fetch, term,
+                walkRow<T, S>(
+                    c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap)), n, sub, packEntry(t, kCentreSlot), fetch, term,
                     [&]() { rho.fold(); });
                 rho.fold();
             }
@@ -456,8 +457,8 @@ namespace sph
                     }
                 };
                 uint32_t const n = min(c.lists.rowLen[t], c.lists.cap);
-                walkRow<S>(
-                    c.lists.list + size_t(t) * c.lists.cap, n, sub, packEntry(t, kCentreSlot), fetch, term, fold);
+                walkRow<T, S>(
+                    c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap)), n, sub, packEntry(t, kCentreSlot), fetch, term, fold);
             }
             ForceSums s{};
             s.a[0] = laneSum<S>(A.ax.value());

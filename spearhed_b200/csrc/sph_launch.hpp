@@ -162,17 +162,45 @@ namespace sph
         uint32_t* bend;
     };
 
-    //! Neighbour lists: row t (sorted target index) starts at list[t * cap] and
-    //! holds rowLen[t] entries packEntry(j, stencil slot).
-    //! The pair passes load rows in groups of 16 entries: the last row's group
-    //! may reach this far past the array's end.
-    constexpr uint32_t kRowSlack = 16;
+    //! Neighbour lists: row t (sorted target index) holds rowLen[t] entries
+    //! packEntry(j, stencil slot); entry k is at
+    //! list[rowStart<T>(t, cap) + rowPlace<T>(k)], T the pair precision.
+    //!
+    //! FP32: the rows of four consecutive targets are interleaved in octets (a
+    //! 128-byte line holds eight entries of each).  A pair pass's lanes, consecutive
+    //! targets at about the same k, then read a quad of entries from 8 lines, not
+    //! 32; the neighbour build's stores touch more lines for it.  Steps, rows
+    //! contiguous -> interleaved, ms: Kelvin-Helmholtz 1.35 M 2.365 -> 2.286, rotor
+    //! 0.9 M 1.706 -> 1.664, Brio-Wu 2 M 2.594 -> 2.549, Sod 18 k 0.205 -> 0.207.
+    //! FP64: contiguous rows; two lanes share a target there and the interleaved
+    //! rows cost the build more than they give (Brio-Wu 176 k 0.611 -> 0.625).
+    template<typename T, typename I>
+    __device__ __forceinline__ I rowStart(I t, I cap)
+    {
+        if constexpr(sizeof(T) == 4)
+            return (t >> 2) * (I(4) * cap) + (t & I(3)) * I(8);
+        else
+            return t * cap;
+    }
+    template<typename T>
+    __device__ __forceinline__ uint32_t rowPlace(uint32_t k)
+    {
+        if constexpr(sizeof(T) == 4)
+            return k + (k >> 3) * 24u;
+        else
+            return k;
+    }
+    //! Words of the lists of n targets.
+    inline size_t listWords(size_t n, size_t cap)
+    {
+        return ((n + 3) & ~size_t(3)) * cap;
+    }
     struct Lists
     {
         uint32_t* list;
         uint32_t* count;
         uint32_t* rowLen; //!< entries of the row the pair passes read (0 for rows not built)
-        uint32_t cap;
+        uint32_t cap; //!< entries per row, a multiple of 8
     };
 
     //! Scalars the step keeps on the device so a step never waits for the host.
