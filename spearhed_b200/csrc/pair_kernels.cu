@@ -98,6 +98,54 @@ namespace sph
             fold();
         }
 
+        //! A source's position with its stencil image's shift added.
+        //!
+        //! FP32: the slot's offsets o in {-1, 0, 1} are worked out in floats (slot s =
+        //! (o0 + 1) + 3 (o1 + 1) + 9 (o2 + 1), so o2 = round((s - 13)/9) and so on; no
+        //! quotient comes within 0.05 of a half) and the shift o e is an exact
+        //! product, so the fused add rounds like the sum with the shift table's
+        //! entry.  Reading the table per entry went through the gathers' own
+        //! bottleneck: 6 of 18 (density) and 47 (force) L1 wavefronts per entry, for
+        //! 6 instructions saved; offsets read from constant memory were slower still
+        //! (density pass 0.51 ms against 0.23: divergent constant reads serialise).
+        //! FP64, not bound by the L1, reads the table.
+        template<typename T>
+        struct ImageShift;
+        template<>
+        struct ImageShift<float>
+        {
+            float e0, e1, e2;
+            __device__ __forceinline__ ImageShift(DevCtx const& c, int box)
+                : e0(c.boxes[box].edgef[0])
+                , e1(c.boxes[box].edgef[1])
+                , e2(c.boxes[box].edgef[2])
+            {
+            }
+            __device__ __forceinline__ float4 at(float4 p, uint32_t entry) const
+            {
+                constexpr float kRound = 12582912.f; // 1.5 2^23: adding it rounds to an integer
+                float const s = __uint_as_float((entry & 31u) | 0x4b000000u) - (8388608.f + float(kCentreSlot));
+                float const oz = __fmaf_rn(s, 1.f / 9.f, kRound) - kRound;
+                float const r = __fmaf_rn(oz, -9.f, s);
+                float const oy = __fmaf_rn(r, 1.f / 3.f, kRound) - kRound;
+                float const ox = __fmaf_rn(oy, -3.f, r);
+                return make_float4(__fmaf_rn(ox, e0, p.x), __fmaf_rn(oy, e1, p.y), __fmaf_rn(oz, e2, p.z), p.w);
+            }
+        };
+        template<>
+        struct ImageShift<double>
+        {
+            D4 const* table;
+            __device__ __forceinline__ ImageShift(DevCtx const& c, int box) : table(shiftTable<double>(c, box))
+            {
+            }
+            __device__ __forceinline__ D4 at(D4 p, uint32_t entry) const
+            {
+                D4 const o = ld4(table + (entry & 31u));
+                return D4{p.x + o.x, p.y + o.y, p.z + o.z, p.w};
+            }
+        };
+
         //! Sum over the lanes of a target (every lane gets it).
         template<int S>
         __device__ __forceinline__ double laneSum(double v)
@@ -161,26 +209,25 @@ namespace sph
             {
                 V4 const own = ld4(rec.pm + t);
                 HConst<T> const hk = hconst<K, T>(rec.hc[t]);
-                V4 const* const stab = shiftTable<T>(c, myBox);
+                ImageShift<T> const shift(c, myBox);
                 if(sub == 0)
                     rho.add(own.w * kernelW<K, T>(T(0), hk));
                 V4 npm{};
-                uint32_t nslot = 0;
+                uint32_t entry = 0; // the fetched one
                 auto fetch = [&](uint32_t e)
                 {
                     if(!checkIndex((e >> 5) < c.n, c.status, kChkRowEntry))
                         e = 0;
-                    nslot = e & 31u;
+                    entry = e;
                     npm = ld4(rec.pm + (e >> 5));
                 };
                 auto term = [&](uint32_t next)
                 {
-                    V4 const pj = npm;
-                    V4 const o = ld4(stab + nslot);
+                    V4 const pj = shift.at(npm, entry);
                     fetch(next);
-                    T const dx = own.x - (pj.x + o.x);
-                    T const dy = own.y - (pj.y + o.y);
-                    T const dz = own.z - (pj.z + o.z);
+                    T const dx = own.x - pj.x;
+                    T const dy = own.y - pj.y;
+                    T const dz = own.z - pj.z;
                     T const r2 = dx * dx + dy * dy + dz * dz;
                     rho.add(pj.w * kernelW<K, T>(r2 * invDistance(r2), hk));
                 };
@@ -259,8 +306,8 @@ namespace sph
             return o;
         }
 
-        //! One pair term of the force pass: source records pj, vj, tj, bj and
-        //! the source's stencil image shift sh.
+        //! One pair term of the force pass: source records pj (shifted to its
+        //! image), vj, tj, bj.
         template<int K, typename T, int PH, typename V4>
         __device__ __forceinline__ void pairTerm(
             OwnTarget<V4, T> const& ow,
@@ -268,16 +315,15 @@ namespace sph
             V4 const& pj,
             V4 const& vj,
             V4 const& tj,
-            V4 const& bj,
-            V4 const& sh)
+            V4 const& bj)
         {
             V4 const& pi = ow.pi;
             V4 const& vi = ow.vi;
             V4 const& ti = ow.ti;
             V4 const& bi = ow.bi;
-            T const rx = pi.x - (pj.x + sh.x);
-            T const ry = pi.y - (pj.y + sh.y);
-            T const rz = pi.z - (pj.z + sh.z);
+            T const rx = pi.x - pj.x;
+            T const ry = pi.y - pj.y;
+            T const rz = pi.z - pj.z;
             T const r2 = rx * rx + ry * ry + rz * rz;
             T const invR = invDistance(r2);
             T const r = r2 * invR;
@@ -417,16 +463,16 @@ namespace sph
             if(act)
             {
                 OwnTarget<V4, T> const own = loadOwn<K, T, PH>(rec, pa, t);
-                V4 const* const stab = shiftTable<T>(c, myBox);
+                ImageShift<T> const shift(c, myBox);
                 A.vsig = own.ti.z;
                 V4 npm{}, nfv{}, nft{}, nfb{};
-                uint32_t nslot = 0;
+                uint32_t entry = 0; // the fetched one
                 auto fetch = [&](uint32_t e)
                 {
                     if(!checkIndex((e >> 5) < c.n, c.status, kChkRowEntry))
                         e = 0;
                     uint32_t const j = e >> 5;
-                    nslot = e & 31u;
+                    entry = e;
                     npm = ld4(rec.pm + j);
                     nfv = ld4(rec.fv + j);
                     nft = ld4(rec.ft + j);
@@ -435,10 +481,9 @@ namespace sph
                 };
                 auto term = [&](uint32_t next)
                 {
-                    V4 const pj = npm, vj = nfv, tj = nft, bj = nfb;
-                    V4 const o = ld4(stab + nslot);
+                    V4 const pj = shift.at(npm, entry), vj = nfv, tj = nft, bj = nfb;
                     fetch(next);
-                    pairTerm<K, T, PH>(own, A, pj, vj, tj, bj, o);
+                    pairTerm<K, T, PH>(own, A, pj, vj, tj, bj);
                 };
                 auto fold = [&]()
                 {
