@@ -411,6 +411,7 @@ namespace sph
             uint32_t const parts = 1u << partShift;
             uint32_t const nWork = *c.activeTotal << partShift;
             uint32_t pending = 0;
+            int box = 0; // items come in ascending order, so the box only moves up
             if(lane == 0)
                 pending = atomicAdd(c.work, 1u);
             for(uint32_t q = __shfl_sync(0xffffffffu, pending, 0); q < nWork; q = __shfl_sync(0xffffffffu, pending, 0))
@@ -418,7 +419,8 @@ namespace sph
                 if(lane == 0)
                     pending = atomicAdd(c.work, 1u);
                 uint32_t const item = q >> partShift;
-                int const box = boxOfWork(c.boxes, c.nbox, item);
+                if(item - c.boxes[box].activeBase >= c.boxes[box].nItems)
+                    box = boxOfWork(c.boxes, c.nbox, item);
                 // item -> cell: the box's level-0 cells first, then its level-1 cells
                 uint32_t const l = item - c.boxes[box].activeBase;
                 uint32_t const nc0 = c.boxes[box].ncells;
@@ -440,12 +442,13 @@ namespace sph
                 int ct[3], c0[3];
                 {
                     uint32_t const li = lt ? l - B.ncells : l;
-                    uint32_t const par = lt ? li / B.msub : li;
+                    uint32_t const par = lt ? li >> __popc(B.msub - 1u) : li; // msub is 2, 4 or 8
                     uint32_t const n0 = uint32_t(B.n[0]), n1 = uint32_t(B.n[1]);
-                    c0[0] = int(par % n0);
-                    c0[1] = int((par / n0) % n1);
-                    c0[2] = int(par / (n0 * n1));
-                    uint32_t sub = lt ? li - par * B.msub : 0u;
+                    uint32_t const row = par / n0, plane = row / n1;
+                    c0[0] = int(par - row * n0);
+                    c0[1] = int(row - plane * n1);
+                    c0[2] = int(plane);
+                    uint32_t sub = lt ? li & (B.msub - 1u) : 0u;
 #pragma unroll
                     for(int a = 0; a < 3; ++a)
                     {
@@ -507,21 +510,15 @@ namespace sph
                             int const n1 = n0 << sh;
                             int const fa = ct[a] + off[a];
                             o[a] = (fa >> sh) - c0[a];
-                            f[a] = fa < 0 || fa >= n1 ? (B.periodic[a] ? (fa + n1) % n1 : -1) : fa;
-                            ok = ok && f[a] >= 0;
+                            f[a] = fa < 0 ? fa + n1 : (fa >= n1 ? fa - n1 : fa);
+                            ok = ok && (f[a] == fa || B.periodic[a]);
                         }
                         else
                         {
                             o[a] = off[a];
-                            int ca = c0[a] + o[a];
-                            if(ca < 0 || ca >= n0)
-                            {
-                                if(B.periodic[a])
-                                    ca = (ca + n0) % n0;
-                                else
-                                    ok = false;
-                            }
-                            f[a] = ca;
+                            int const ca = c0[a] + o[a];
+                            f[a] = ca < 0 ? ca + n0 : (ca >= n0 ? ca - n0 : ca);
+                            ok = ok && (f[a] == ca || B.periodic[a]);
                         }
                     }
                     slot = uint32_t((o[0] + 1) + 3 * (o[1] + 1) + 9 * (o[2] + 1));
@@ -617,8 +614,8 @@ namespace sph
                         {
                             T const l0 = A.act ? ax[a] : inf, l1 = Bc.act ? bx[a] : inf;
                             T const h0 = A.act ? ax[a] : -inf, h1 = Bc.act ? bx[a] : -inf;
-                            bLo[a] = warpMinT<T>(l0 < l1 ? l0 : l1);
-                            bHi[a] = warpMaxT<T>(h0 > h1 ? h0 : h1);
+                            bLo[a] = warpMinT(l0 < l1 ? l0 : l1);
+                            bHi[a] = warpMaxT(h0 > h1 ? h0 : h1);
                         }
                     }
                     T const widen = T(1) + T(1.0 / 1024.0);
@@ -627,7 +624,7 @@ namespace sph
                     if constexpr(PAIRMAX)
                     {
                         T const nA = A.act ? A.nR2 : T(0), nB = Bc.act ? Bc.nR2 : T(0);
-                        nRt = warpMinT<T>(nA < nB ? nA : nB);
+                        nRt = warpMinT(nA < nB ? nA : nB);
                     }
                     // The page of 32 descriptors being staged; page 0 (all of a
                     // single-level box's 27 slots) was described for the cell.

@@ -284,8 +284,8 @@ namespace
 #pragma unroll
                 for(int a = 0; a < 3; ++a)
                 {
-                    bLo[a] = sph::warpMinT<T>(act ? x[a] : T(1e30f));
-                    bHi[a] = sph::warpMaxT<T>(act ? x[a] : T(-1e30f));
+                    bLo[a] = sph::warpMinT(act ? x[a] : T(1e30f));
+                    bHi[a] = sph::warpMaxT(act ? x[a] : T(-1e30f));
                 }
                 // rounding is monotone, so with the radius widened by 2^-10 the box
                 // test passes every candidate that the exact test accepts

@@ -244,26 +244,26 @@ namespace sph
         return v;
     }
 
-    template<typename T>
-    __device__ __forceinline__ T warpMinT(T v)
+    //! Minimum and maximum over the warp (FP32: one sm_100 reduction instruction
+    //! instead of five shuffles and compares).
+    __device__ __forceinline__ float warpMinT(float v)
     {
-#pragma unroll
-        for(int o = 16; o > 0; o >>= 1)
-        {
-            T const w = __shfl_xor_sync(0xffffffffu, v, o);
-            v = w < v ? w : v;
-        }
-        return v;
+        float r;
+        asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+        return r;
     }
-    template<typename T>
-    __device__ __forceinline__ T warpMaxT(T v)
+    __device__ __forceinline__ float warpMaxT(float v)
     {
-#pragma unroll
-        for(int o = 16; o > 0; o >>= 1)
-        {
-            T const w = __shfl_xor_sync(0xffffffffu, v, o);
-            v = w > v ? w : v;
-        }
-        return v;
+        float r;
+        asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+        return r;
+    }
+    __device__ __forceinline__ double warpMinT(double v)
+    {
+        return warpMinD(v);
+    }
+    __device__ __forceinline__ double warpMaxT(double v)
+    {
+        return warpMaxD(v);
     }
 } // namespace sph
