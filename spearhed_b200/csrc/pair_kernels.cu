@@ -98,6 +98,64 @@ namespace sph
             fold();
         }
 
+        //! Lanes per target of the FP32 passes on small systems: each takes blocks of
+        //! 8 consecutive entries, and the blocks' partial sums are folded in row
+        //! order by every lane (foldBlocks), so the sums, to the bit, are those of one
+        //! lane walking the whole row.
+        constexpr int kWide = 8;
+
+        //! Folds the lanes' block partials, in block order, into each lane's sum.
+        __device__ __forceinline__ void foldBlocks(Acc<float>& a, int blocks, uint32_t lanes)
+        {
+            for(int s = 0; s < blocks; ++s)
+                a.c.fold(__shfl_sync(lanes, a.part, s, kWide));
+            a.part = 0.f;
+        }
+
+        //! Walks a row with kWide lanes: lane s takes the blocks s, s + 8, ... of 8
+        //! entries; foldAll(blocks, lanes) closes each round of up to 8 blocks.
+        template<typename F, typename M, typename D>
+        __device__ __forceinline__ void walkRowWide(
+            uint32_t const* row,
+            uint32_t n,
+            uint32_t sub,
+            uint32_t any,
+            F&& fetch,
+            M&& term,
+            D&& foldAll)
+        {
+            uint32_t const lanes = 0xffu << (threadIdx.x & 24u);
+            for(uint32_t base = 0; base < n; base += 8 * kWide)
+            {
+                uint32_t const k = base + 8 * sub;
+                if(k < n)
+                {
+                    uint4 const* const q = reinterpret_cast<uint4 const*>(row + rowPlace<float>(k));
+                    uint4 const a = q[0], b = q[1];
+                    uint32_t const m = n - k;
+                    fetch(a.x);
+                    term(m > 1 ? a.y : any);
+                    if(m > 1)
+                        term(m > 2 ? a.z : any);
+                    if(m > 2)
+                        term(m > 3 ? a.w : any);
+                    if(m > 3)
+                        term(m > 4 ? b.x : any);
+                    if(m > 4)
+                        term(m > 5 ? b.y : any);
+                    if(m > 5)
+                        term(m > 6 ? b.z : any);
+                    if(m > 6)
+                        term(m > 7 ? b.w : any);
+                    if(m > 7)
+                        term(any);
+                }
+                __syncwarp(lanes);
+                uint32_t const left = (n - base + 7) / 8;
+                foldAll(int(left < kWide ? left : kWide), lanes);
+            }
+        }
+
         //! A source's position with its stencil image's shift added.
         //!
         //! FP32: the slot's offsets o in {-1, 0, 1} are worked out in floats (slot s =
@@ -192,12 +250,12 @@ namespace sph
         //! its own, beside the neighbour build: its lanes all have work (the
         //! build's warps hold one cell each), and neither kernel carries the
         //! other's registers and instructions.
-        template<int K, typename T>
+        template<int K, typename T, bool kSmall>
         __global__ void __launch_bounds__(kThreads) kDensity(DevCtx c, PhysArgs pa)
         {
             using V4 = typename PairCfg<T>::V4;
             Records<V4, T> const rec = records<T>(c);
-            constexpr int S = kLanes<T>;
+            constexpr int S = kSmall ? kWide : kLanes<T>;
             uint32_t const sub = threadIdx.x & uint32_t(S - 1);
             uint32_t const t = (blockIdx.x * kThreads + threadIdx.x) / S;
             if(blockIdx.x == 0 && threadIdx.x == 0)
@@ -228,16 +286,27 @@ namespace sph
                     T const dx = own.x - pj.x;
                     T const dy = own.y - pj.y;
                     T const dz = own.z - pj.z;
-                    T const r2 = dx * dx + dy * dy + dz * dz;
+                    T const r2 = dot3(dx, dy, dz, dx, dy, dz);
                     rho.add(pj.w * kernelW<K, T>(r2 * invDistance(r2), hk));
                 };
                 uint32_t const n = min(c.lists.rowLen[t], c.lists.cap);
-                walkRow<T, S>(
-                    c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap)), n, sub, packEntry(t, kCentreSlot), fetch, term,
-                    [&]() { rho.fold(); });
-                rho.fold();
+                uint32_t const* const row = c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap));
+                uint32_t const any = packEntry(t, kCentreSlot);
+                if constexpr(kSmall)
+                {
+                    walkRowWide(
+                        row, n, sub, any, fetch, term,
+                        [&](int blocks, uint32_t lanes) { foldBlocks(rho, blocks, lanes); });
+                    if(n == 0)
+                        foldBlocks(rho, 1, 0xffu << (threadIdx.x & 24u)); // the self term alone
+                }
+                else
+                {
+                    walkRow<T, S>(row, n, sub, any, fetch, term, [&]() { rho.fold(); });
+                    rho.fold();
+                }
             }
-            double const rhoD = laneSum<S>(rho.value());
+            double const rhoD = kSmall ? rho.value() : laneSum<S>(rho.value());
             double ch = 0.0;
             if(act && sub == 0)
             {
@@ -324,7 +393,7 @@ namespace sph
             T const rx = pi.x - pj.x;
             T const ry = pi.y - pj.y;
             T const rz = pi.z - pj.z;
-            T const r2 = rx * rx + ry * ry + rz * rz;
+            T const r2 = dot3(rx, ry, rz, rx, ry, rz);
             T const invR = invDistance(r2);
             T const r = r2 * invR;
             T const si = slopeOverR<K>(r, invR, ow.hk);
@@ -333,10 +402,10 @@ namespace sph
                 sj = slopeOverR<K>(r, invR, hconstFromInv<K, T>(rcpT(vj.w)));
             T const mj = pj.w;
             T const vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
-            T const vr = vx * rx + vy * ry + vz * rz;
+            T const vr = dot3(vx, vy, vz, rx, ry, rz);
             T const msi = mj * si;
             // Isotropic pressure gradient (HydroForces.hpp:155-166).
-            T f = -mj * (ti.y * si + tj.y * sj);
+            T f = -mj * fmaT(ti.y, si, tj.y * sj);
             T const cb = ow.hc + T(0.5) * tj.z; // mean signal speed
             if(ow.av)
             {
@@ -345,7 +414,7 @@ namespace sph
                 T const hb = ow.hh + T(0.5) * vj.w;
                 T const mu = hb * vn * rcpT(r2 + ow.eps * hb * hb);
                 // Pi_ij (s_i + s_j)/2: the halves of the means 1/rho_ij and s_ij cancel
-                T const Pi = mu * (ow.beta * mu - ow.alpha * cb) * rcpT(ti.x + tj.x);
+                T const Pi = mu * fmaT(ow.beta, mu, -ow.alpha * cb) * rcpT(ti.x + tj.x);
                 T const g = mj * Pi * (si + sj);
                 f -= g;
                 A.duav.add(g * vr); // twice the heating
@@ -353,37 +422,37 @@ namespace sph
             T fx = f * rx, fy = f * ry, fz = f * rz;
             A.D.add(msi * vr);
             T const w = vr * invR;
-            T const vs = T(2) * cb - ow.beta * (w < T(0) ? w : T(0));
+            T const vs = fmaT(-ow.beta, w < T(0) ? w : T(0), T(2) * cb);
             A.vsig = vs > A.vsig ? vs : A.vsig;
             if constexpr(PH >= 2)
             {
                 T const dBx = bj.x - bi.x, dBy = bj.y - bi.y, dBz = bj.z - bi.z;
-                T const Bir = bi.x * rx + bi.y * ry + bi.z * rz;
-                T const dBr = dBx * rx + dBy * ry + dBz * rz;
+                T const Bir = dot3(bi.x, bi.y, bi.z, rx, ry, rz);
+                T const dBr = dot3(dBx, dBy, dBz, rx, ry, rz);
                 T const cj = mj * tj.w * sj * (Bir + dBr);
                 if(ow.tensile)
                 {
                     // stress + Borve: c_i B_i + c_j B_j - B_i (c_i + c_j) = c_j (B_j - B_i)
-                    fx += cj * dBx;
-                    fy += cj * dBy;
-                    fz += cj * dBz;
+                    fx = fmaT(cj, dBx, fx);
+                    fy = fmaT(cj, dBy, fy);
+                    fz = fmaT(cj, dBz, fz);
                 }
                 else
                 {
                     T const ci = msi * Bir * ti.w;
-                    fx += ci * bi.x + cj * bj.x;
-                    fy += ci * bi.y + cj * bj.y;
-                    fz += ci * bi.z + cj * bj.z;
+                    fx = fmaT(cj, bj.x, fmaT(ci, bi.x, fx));
+                    fy = fmaT(cj, bj.y, fmaT(ci, bi.y, fy));
+                    fz = fmaT(cj, bj.z, fmaT(ci, bi.z, fz));
                 }
                 T const wB = msi * Bir;
                 T gx = wB * vx, gy = wB * vy, gz = wB * vz;
                 if(ow.dedner)
                 {
                     // rho_i^2 * m_j (psi_i/rho_i^2 s_i + psi_j/rho_j^2 s_j) r
-                    T const g = ow.rho2i * mj * (bi.w * si + bj.w * sj);
-                    gx += g * rx;
-                    gy += g * ry;
-                    gz += g * rz;
+                    T const g = ow.rho2i * mj * fmaT(bi.w, si, bj.w * sj);
+                    gx = fmaT(g, rx, gx);
+                    gy = fmaT(g, ry, gy);
+                    gz = fmaT(g, rz, gz);
                 }
                 A.tx.add(gx);
                 A.ty.add(gy);
@@ -445,13 +514,13 @@ namespace sph
 
         //! Force pass; the records of the next entry are in flight while the
         //! current one is used.
-        template<int K, typename T, int PH, int MINB>
+        template<int K, typename T, int PH, int MINB, bool kSmall = false>
         __global__ void __launch_bounds__(kThreads, MINB) kForce(DevCtx c, PhysArgs pa)
         {
             using V4 = typename PairCfg<T>::V4;
             constexpr bool kMhd = PH >= 2;
             Records<V4, T> const rec = records<T>(c);
-            constexpr int S = kLanes<T>;
+            constexpr int S = kSmall ? kWide : kLanes<T>;
             uint32_t const sub = threadIdx.x & uint32_t(S - 1);
             uint32_t const t = (blockIdx.x * kThreads + threadIdx.x) / S;
             bool const act = t < c.n && isTarget(c.cur.role[t]);
@@ -502,22 +571,45 @@ namespace sph
                     }
                 };
                 uint32_t const n = min(c.lists.rowLen[t], c.lists.cap);
-                walkRow<T, S>(
-                    c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap)), n, sub, packEntry(t, kCentreSlot), fetch, term, fold);
+                uint32_t const* const row = c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap));
+                uint32_t const any = packEntry(t, kCentreSlot);
+                if constexpr(kSmall)
+                    walkRowWide(
+                        row, n, sub, any, fetch, term,
+                        [&](int blocks, uint32_t lanes)
+                        {
+                            foldBlocks(A.ax, blocks, lanes);
+                            foldBlocks(A.ay, blocks, lanes);
+                            foldBlocks(A.az, blocks, lanes);
+                            foldBlocks(A.D, blocks, lanes);
+                            if(av)
+                                foldBlocks(A.duav, blocks, lanes);
+                            if constexpr(kMhd)
+                            {
+                                foldBlocks(A.tx, blocks, lanes);
+                                foldBlocks(A.ty, blocks, lanes);
+                                foldBlocks(A.tz, blocks, lanes);
+                                foldBlocks(A.divb, blocks, lanes);
+                            }
+                        });
+                else
+                    walkRow<T, S>(row, n, sub, any, fetch, term, fold);
             }
+            // kSmall: every lane holds the folded sums already
+            constexpr int kSum = kSmall ? 1 : S;
             ForceSums s{};
-            s.a[0] = laneSum<S>(A.ax.value());
-            s.a[1] = laneSum<S>(A.ay.value());
-            s.a[2] = laneSum<S>(A.az.value());
-            s.D = laneSum<S>(A.D.value());
+            s.a[0] = laneSum<kSum>(A.ax.value());
+            s.a[1] = laneSum<kSum>(A.ay.value());
+            s.a[2] = laneSum<kSum>(A.az.value());
+            s.D = laneSum<kSum>(A.D.value());
             if(av)
-                s.duav = 0.5 * laneSum<S>(A.duav.value());
+                s.duav = 0.5 * laneSum<kSum>(A.duav.value());
             if constexpr(kMhd)
             {
-                s.t[0] = laneSum<S>(A.tx.value());
-                s.t[1] = laneSum<S>(A.ty.value());
-                s.t[2] = laneSum<S>(A.tz.value());
-                s.divb = -laneSum<S>(A.divb.value());
+                s.t[0] = laneSum<kSum>(A.tx.value());
+                s.t[1] = laneSum<kSum>(A.ty.value());
+                s.t[2] = laneSum<kSum>(A.tz.value());
+                s.divb = -laneSum<kSum>(A.divb.value());
             }
 #pragma unroll
             for(int o = 1; o < S; o <<= 1)
@@ -537,12 +629,22 @@ namespace sph
         // FP64: 3.  Variant 0 is the default.
         constexpr int kForceVariants32 = 2, kForceVariants64 = 1;
 
-        //! Blocks of a pass over the targets: kLanes threads each.
-        template<typename T>
-        unsigned rowBlocks(DevCtx const& c)
+        //! Blocks of a pass with this many lanes per target.
+        unsigned rowBlocks(DevCtx const& c, int lanes)
         {
-            return unsigned((uint64_t(c.n) * kLanes<T> + kThreads - 1) / kThreads);
+            return unsigned((uint64_t(c.n) * uint64_t(lanes) + kThreads - 1) / kThreads);
         }
+
+        //! Particle counts up to which the FP32 passes use kWide lanes per target:
+        //! below them one lane per target leaves most warp slots empty and the pass
+        //! waits for its longest row.  The fold of every block by every lane costs
+        //! 8 x 8 instructions per sum and round, so the line lies lower the more sums
+        //! a pass has.  One lane -> eight, ms: density Sod 2.3 k 0.064 -> 0.051 (with
+        //! the neighbour build), 18 k 0.103 -> 0.090, 36 k 0.098 -> 0.090, Orszag-Tang
+        //! 37 k 0.085 -> 0.082, 66 k 0.111 -> 0.117; hydro force Sod 2.3 k 0.029 -> 0.015,
+        //! 18 k 0.031 -> 0.025, 36 k 0.033 -> 0.038; SPMHD force Orszag-Tang 6.4 k
+        //! 0.028 -> 0.020, 16 k 0.028 -> 0.035.
+        constexpr uint32_t kWideDensity = 148 * 256, kWideHydro = 148 * 128, kWideMhd = 148 * 64;
 
         template<int K, typename T, int PH>
         void forceLaunch(DevCtx const& c, PhysArgs const& pa, int variant, cudaStream_t s)
@@ -553,13 +655,15 @@ namespace sph
             {
                 // variant 0: SPMHD 4 blocks/SM (128 registers), hydro 5; variant 1 the other
                 constexpr int a = PH >= 2 ? 4 : 5, b = PH >= 2 ? 5 : 4;
-                if(variant == 1)
-                    kForce<K, T, PH, b><<<rowBlocks<T>(c), kThreads, 0, s>>>(c, pa);
+                if(c.n <= (PH >= 2 ? kWideMhd : kWideHydro))
+                    kForce<K, T, PH, a, true><<<rowBlocks(c, kWide), kThreads, 0, s>>>(c, pa);
+                else if(variant == 1)
+                    kForce<K, T, PH, b><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
                 else
-                    kForce<K, T, PH, a><<<rowBlocks<T>(c), kThreads, 0, s>>>(c, pa);
+                    kForce<K, T, PH, a><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
             }
             else
-                kForce<K, T, PH, 3><<<rowBlocks<T>(c), kThreads, 0, s>>>(c, pa);
+                kForce<K, T, PH, 3><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
             countLaunches(1);
         }
 
@@ -582,7 +686,10 @@ namespace sph
         {
             if(!c.n)
                 return;
-            kDensity<K, T><<<rowBlocks<T>(c), kThreads, 0, s>>>(c, pa);
+            if(sizeof(T) == 4 && c.n <= kWideDensity)
+                kDensity<K, float, true><<<rowBlocks(c, kWide), kThreads, 0, s>>>(c, pa);
+            else
+                kDensity<K, T, false><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
             countLaunches(1);
         }
 
@@ -618,6 +725,7 @@ namespace sph
         template<int K, int PH>
         void configureForceK()
         {
+            preferL1(kForce<K, float, PH, PH >= 2 ? 4 : 5, true>);
             preferL1(kForce<K, float, PH, 4>);
             preferL1(kForce<K, float, PH, 5>);
             preferL1(kForce<K, double, PH, 3>);
@@ -626,8 +734,9 @@ namespace sph
         template<int K>
         void configureK()
         {
-            preferL1(kDensity<K, float>);
-            preferL1(kDensity<K, double>);
+            preferL1(kDensity<K, float, false>);
+            preferL1(kDensity<K, float, true>);
+            preferL1(kDensity<K, double, false>);
             configureForceK<K, 0>();
             configureForceK<K, 1>();
             configureForceK<K, 2>();

@@ -100,6 +100,24 @@ namespace sph
     }
     constexpr uint32_t kMaxParticles = 1u << 27;
 
+    //! a b + c, rounded once.  Sums of two products are written with it: the
+    //! compiler would fuse one of the two, which one varying from one copy of the
+    //! code to the next, and with it the last bit.
+    __device__ __forceinline__ float fmaT(float a, float b, float c)
+    {
+        return __fmaf_rn(a, b, c);
+    }
+    __device__ __forceinline__ double fmaT(double a, double b, double c)
+    {
+        return __fma_rn(a, b, c);
+    }
+    //! a . b, fused in x, y, z order.
+    template<typename T>
+    __device__ __forceinline__ T dot3(T ax, T ay, T az, T bx, T by, T bz)
+    {
+        return fmaT(az, bz, fmaT(ay, by, ax * bx));
+    }
+
     // --------------------------------------------------------------- kernels
     // Kernel functions follow the reference's formulas
     // (include/spearhed/sph/CubicSplineKernel.hpp:49-140,
@@ -161,9 +179,9 @@ namespace sph
             T const a = T(3) - x, b = T(2) - x, c = T(1) - x;
             T const a2 = a * a, b2 = b * b, c2 = c * c;
             if(x < T(1))
-                return a2 * a2 * a - T(6) * b2 * b2 * b + T(15) * c2 * c2 * c;
+                return fmaT(T(15) * c2 * c2, c, fmaT(T(-6) * b2 * b2, b, a2 * a2 * a));
             if(x < T(2))
-                return a2 * a2 * a - T(6) * b2 * b2 * b;
+                return fmaT(T(-6) * b2 * b2, b, a2 * a2 * a);
             if(x < T(3))
                 return a2 * a2 * a;
             return T(0);
@@ -174,9 +192,9 @@ namespace sph
             T const a = T(3) - x, b = T(2) - x, c = T(1) - x;
             T const a2 = a * a, b2 = b * b, c2 = c * c;
             if(x < T(1))
-                return T(-5) * a2 * a2 + T(30) * b2 * b2 - T(75) * c2 * c2;
+                return fmaT(T(-75) * c2, c2, fmaT(T(30) * b2, b2, T(-5) * a2 * a2));
             if(x < T(2))
-                return T(-5) * a2 * a2 + T(30) * b2 * b2;
+                return fmaT(T(30) * b2, b2, T(-5) * a2 * a2);
             if(x < T(3))
                 return T(-5) * a2 * a2;
             return T(0);

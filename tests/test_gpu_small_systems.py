@@ -1,0 +1,38 @@
+"""The FP32 pair passes of small systems (up to 37,888 particles for the density,
+18,944 and 9,472 for the hydro and SPMHD forces) give every target eight lanes.
+The sums are folded in row order, so the same box must get the same bits alone
+(eight lanes) and inside an ensemble above the limits (one lane).
+"""
+import numpy as np
+import pytest
+
+from spearhed_b200 import abi, setups
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("pos", "vel", "u", "density", "h", "B", "psi", "dvdt", "dudt", "dBdt", "dpsidt", "divB")
+
+
+def _run(w, steps=3):
+    import spearhed_b200 as sb
+    with sb.context_for(w) as ctx:
+        ctx.step(steps)
+        return ctx.get_species(abi.SPECIES_DEFAULT)
+
+
+@pytest.mark.parametrize("physics", ["mhd", "hydro_av"])
+def test_a_small_box_gets_the_bits_of_the_large_ensemble(physics):
+    kw = dict(nbox=8, n_lo=4096, n_hi=16384)
+    every = setups.brio_wu_ensemble(**kw)
+    n = np.bincount(every.species[abi.SPECIES_DEFAULT].box_id)
+    assert n.sum() > 37888 and n.min() <= 9472
+    if physics == "hydro_av":
+        every.params.physics &= ~(abi.PHYS_MHD | abi.PHYS_DEDNER | abi.PHYS_TENSILE)
+    whole = _run(every)
+    of_box = every.species[abi.SPECIES_DEFAULT].box_id
+    for b in (int(np.argmin(n)), int(np.argsort(n)[len(n) // 2])):
+        alone = setups.brio_wu_ensemble(**kw, boxes=[b])
+        alone.params.physics = every.params.physics
+        got = _run(alone)
+        for f in FIELDS:
+            assert np.array_equal(getattr(got, f), getattr(whole, f)[..., of_box == b]), (b, f)
