@@ -51,15 +51,23 @@ namespace sph
             int32_t const bx = c.cur.box[p];
             BoxDev const& B = c.boxes[bx];
             double const dt = c.bs.dt[bx];
-            double x[3];
-            bool finite = true;
+            bool const moves = drift && (role & SPH_ROLE_MOVABLE);
+            // every load before the first store: the columns may alias for all the
+            // compiler knows, and a store would hold back the loads that follow it
+            double x[3], v[3];
 #pragma unroll
             for(int a = 0; a < 3; ++a)
             {
                 x[a] = c.cur.x[a][p];
-                if(drift && (role & SPH_ROLE_MOVABLE))
+                v[a] = moves ? c.cur.v[a][p] : 0.0;
+            }
+            bool finite = true;
+#pragma unroll
+            for(int a = 0; a < 3; ++a)
+            {
+                if(moves)
                 {
-                    x[a] = __dadd_rn(x[a], __dmul_rn(c.cur.v[a][p], dt));
+                    x[a] = __dadd_rn(x[a], __dmul_rn(v[a], dt));
                     if(B.periodic[a])
                     {
                         double const hiEdge = B.lo[a] + B.L[a];
@@ -157,6 +165,7 @@ namespace sph
             uint32_t const q = perm[p];
             if(!checkIndex(q < c.n, c.status, kChkPermute))
                 return;
+            // every load before the first store (see kDriftKeys)
             double x[3], v[3], Bv[3];
 #pragma unroll
             for(int a = 0; a < 3; ++a)
@@ -164,20 +173,25 @@ namespace sph
                 x[a] = c.cur.x[a][q];
                 v[a] = c.cur.v[a][q];
                 Bv[a] = c.cur.B[a][q];
+            }
+            double const u = c.cur.u[q], m = c.cur.m[q], h = c.cur.h[q], rho = c.cur.rho[q], psi = c.cur.psi[q];
+            uint32_t const id = c.cur.id[q];
+            int32_t const b = c.cur.box[q];
+            uint8_t const role = c.cur.role[q];
+#pragma unroll
+            for(int a = 0; a < 3; ++a)
+            {
                 c.alt.x[a][p] = x[a];
                 c.alt.v[a][p] = v[a];
                 c.alt.B[a][p] = Bv[a];
             }
-            double const u = c.cur.u[q], m = c.cur.m[q], h = c.cur.h[q], rho = c.cur.rho[q], psi = c.cur.psi[q];
             c.alt.u[p] = u;
             c.alt.m[p] = m;
             c.alt.h[p] = h;
             c.alt.rho[p] = rho;
             c.alt.psi[p] = psi;
-            c.alt.id[p] = c.cur.id[q];
-            int32_t const b = c.cur.box[q];
+            c.alt.id[p] = id;
             c.alt.box[p] = b;
-            uint8_t const role = c.cur.role[q];
             c.alt.role[p] = role;
             // no row until the neighbour build writes one
             c.lists.count[p] = 0xffffffffu;
@@ -297,46 +311,72 @@ namespace sph
             {
                 if(!isTarget(c.cur.role[p]))
                     continue;
-                double const dt = c.bs.dt[c.cur.box[p]];
-                double const m = c.cur.m[p];
+                // every load before the first store (see kDriftKeys): waiting for the
+                // columns one after another took 70 us where their bytes take 37
+                // (Orszag-Tang 1 M)
+                bool const adaptive = pa.physics & SPH_PHYS_ADAPTIVE_H;
+                int32_t const bx = c.cur.box[p];
+                double const m = c.cur.m[p], rho = c.cur.rho[p], u0 = c.cur.u[p], du = c.d.dudt[p];
+                double v[3], a[3], B[3] = {0.0, 0.0, 0.0}, dB[3] = {0.0, 0.0, 0.0};
+                double psi = 0.0, dpsi = 0.0, divB = 0.0, h = 0.0;
+#pragma unroll
+                for(int k = 0; k < 3; ++k)
+                {
+                    v[k] = c.cur.v[k][p];
+                    a[k] = c.d.dvdt[k][p];
+                }
+                if(mhd)
+                {
+#pragma unroll
+                    for(int k = 0; k < 3; ++k)
+                    {
+                        B[k] = c.cur.B[k][p];
+                        dB[k] = c.d.dBdt[k][p];
+                    }
+                    psi = c.cur.psi[p];
+                    dpsi = c.d.dpsidt[p];
+                    divB = c.d.divB[p];
+                    h = c.cur.h[p];
+                }
+                double const dt = c.bs.dt[bx];
                 double v2 = 0.0, B2 = 0.0;
 #pragma unroll
-                for(int a = 0; a < 3; ++a)
+                for(int k = 0; k < 3; ++k)
                 {
                     // unfused, as EulerIntegrate.hpp:45-51 on the reference's CPU path
-                    double const va = __dadd_rn(c.cur.v[a][p], __dmul_rn(c.d.dvdt[a][p], dt));
-                    c.cur.v[a][p] = va;
+                    double const va = __dadd_rn(v[k], __dmul_rn(a[k], dt));
+                    c.cur.v[k][p] = va;
                     v2 += va * va;
-                    acc[3 + a] += m * va;
+                    acc[3 + k] += m * va;
                 }
-                double const u = __dadd_rn(c.cur.u[p], __dmul_rn(c.d.dudt[p], dt));
+                double const u = __dadd_rn(u0, __dmul_rn(du, dt));
                 c.cur.u[p] = u;
                 if(mhd)
                 {
 #pragma unroll
-                    for(int a = 0; a < 3; ++a)
+                    for(int k = 0; k < 3; ++k)
                     {
-                        double const Ba = __dadd_rn(c.cur.B[a][p], __dmul_rn(c.d.dBdt[a][p], dt));
-                        c.cur.B[a][p] = Ba;
+                        double const Ba = __dadd_rn(B[k], __dmul_rn(dB[k], dt));
+                        c.cur.B[k][p] = Ba;
                         B2 += Ba * Ba;
                     }
-                    c.cur.psi[p] = __dadd_rn(c.cur.psi[p], __dmul_rn(c.d.dpsidt[p], dt));
+                    c.cur.psi[p] = __dadd_rn(psi, __dmul_rn(dpsi, dt));
                 }
                 acc[0] += 0.5 * m * v2;
                 acc[1] += m * u;
-                double const rho = c.cur.rho[p];
-                if(pa.physics & SPH_PHYS_ADAPTIVE_H)
+                if(adaptive)
                 {
                     // h for the next step from this step's density, capped by the box's h cap
                     double const hn = pa.hfact * cbrt(m / rho);
-                    double const cap = c.boxes[c.cur.box[p]].hcap;
-                    c.cur.h[p] = hn < cap ? hn : cap;
+                    double const cap = c.boxes[bx].hcap;
+                    h = hn < cap ? hn : cap;
+                    c.cur.h[p] = h;
                 }
                 if(mhd && rho > 0.0)
                     acc[2] += 0.5 * m * B2 / (pa.mu0 * rho);
                 if(mhd && B2 > 0.0)
                 {
-                    double const e = fabs(c.d.divB[p]) * c.cur.h[p] / sqrt(B2);
+                    double const e = fabs(divB) * h / sqrt(B2);
                     acc[6] += e;
                     acc[7] += 1.0;
                     acc[8] = fmax(acc[8], e);
