@@ -15,9 +15,9 @@
 //
 // A pass is bound by latency and launches, not by its bytes (8 B in, 8 B out per
 // key): tiles of a fixed 4096 keys gave 18 k keys 5 blocks (10 us a histogram,
-// 12 us a scatter).  rounds follows the key count, for about 128 tiles up to half
-// a million keys and 16 rounds beyond; with up to kFewTiles tiles the scatter
-// adds the tiles' counts itself and step (2) needs no launch.
+// 12 us a scatter).  rounds follows the key count: about 128 tiles up to kFewKeys
+// keys, where the scatter adds the tiles' counts itself and step (2) needs no
+// launch, then four tiles per SM, then 16 rounds.
 #include "sph_launch.hpp"
 
 namespace sph
@@ -27,10 +27,12 @@ namespace sph
         constexpr int kThreads = 256;
         constexpr uint32_t kMaxRounds = 16;
         constexpr uint32_t kFewTiles = 192;
+        constexpr uint32_t kFewKeys = 1u << 17;
 
         uint32_t tileRounds(uint32_t n)
         {
-            uint32_t const r = n / (128u * kThreads);
+            uint32_t const tiles = n <= kFewKeys ? 128u : 4u * 148u;
+            uint32_t const r = n / (tiles * kThreads);
             return r < 1u ? 1u : (r > kMaxRounds ? kMaxRounds : r);
         }
         uint32_t tileCount(uint32_t n)

@@ -705,21 +705,34 @@ namespace sph
         {
             for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
             {
+                // every load before the first store (see kDriftKeys)
+                double x[3], v[3], B[3];
 #pragma unroll
                 for(int a = 0; a < 3; ++a)
                 {
-                    dst.x[a][i] = src.x[a][i];
-                    dst.v[a][i] = src.v[a][i];
-                    dst.B[a][i] = src.B[a][i];
+                    x[a] = src.x[a][i];
+                    v[a] = src.v[a][i];
+                    B[a] = src.B[a][i];
                 }
-                dst.u[i] = src.u[i];
-                dst.m[i] = src.m[i];
-                dst.h[i] = src.h[i];
-                dst.rho[i] = src.rho[i];
-                dst.psi[i] = src.psi[i];
-                dst.id[i] = src.id[i];
-                dst.box[i] = src.box[i];
-                dst.role[i] = src.role[i];
+                double const u = src.u[i], m = src.m[i], h = src.h[i], rho = src.rho[i], psi = src.psi[i];
+                uint32_t const id = src.id[i];
+                int32_t const box = src.box[i];
+                uint8_t const role = src.role[i];
+#pragma unroll
+                for(int a = 0; a < 3; ++a)
+                {
+                    dst.x[a][i] = x[a];
+                    dst.v[a][i] = v[a];
+                    dst.B[a][i] = B[a];
+                }
+                dst.u[i] = u;
+                dst.m[i] = m;
+                dst.h[i] = h;
+                dst.rho[i] = rho;
+                dst.psi[i] = psi;
+                dst.id[i] = id;
+                dst.box[i] = box;
+                dst.role[i] = role;
             }
         }
 
