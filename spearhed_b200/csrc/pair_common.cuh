@@ -188,6 +188,10 @@ namespace sph
         {
             part += x;
         }
+        __device__ __forceinline__ void addProduct(float a, float b)
+        {
+            part = fmaT(a, b, part);
+        }
         __device__ __forceinline__ void fold()
         {
             c.fold(part);
@@ -205,6 +209,10 @@ namespace sph
         __device__ __forceinline__ void add(double x)
         {
             s += x;
+        }
+        __device__ __forceinline__ void addProduct(double a, double b)
+        {
+            s = fmaT(a, b, s);
         }
         __device__ __forceinline__ void fold()
         {

@@ -326,9 +326,9 @@ namespace sph
         //! tensile correction switched at run time, 3 = SPMHD with all three on.
         //!
         //! Accumulators (compensated in FP32): a (pressure, viscosity and magnetic
-        //! force together), D = sum m_j s_i v_ij.r (P dV work, div v and the
-        //! induction's B_i term), the viscous heating, T = sum m_j s_i (B_i.r) v_ij
-        //! + rho_i^2 (Dedner gradient term) for the induction, and the div B sum.
+        //! force together), D = sum m_j s_i v_ij.r (P dV work and div v), the viscous
+        //! heating, T = sum m_j s_i ((B_i.r) v_ij - B_i (v_ij.r)) + rho_i^2 (Dedner
+        //! gradient term) for the induction, and the div B sum.
         //! With the tensile correction the Maxwell-stress force and the Borve term
         //! combine to sum m_j s_j (B_j.r)/(mu0 rho_j^2) (B_j - B_i).
         template<typename T>
@@ -417,10 +417,10 @@ namespace sph
                 T const Pi = mu * fmaT(ow.beta, mu, -ow.alpha * cb) * rcpT(ti.x + tj.x);
                 T const g = mj * Pi * (si + sj);
                 f -= g;
-                A.duav.add(g * vr); // twice the heating
+                A.duav.addProduct(g, vr); // twice the heating
             }
             T fx = f * rx, fy = f * ry, fz = f * rz;
-            A.D.add(msi * vr);
+            A.D.addProduct(msi, vr);
             T const w = vr * invR;
             T const vs = fmaT(-ow.beta, w < T(0) ? w : T(0), T(2) * cb);
             A.vsig = vs > A.vsig ? vs : A.vsig;
@@ -444,20 +444,20 @@ namespace sph
                     fy = fmaT(cj, bj.y, fmaT(ci, bi.y, fy));
                     fz = fmaT(cj, bj.z, fmaT(ci, bi.z, fz));
                 }
-                T const wB = msi * Bir;
-                T gx = wB * vx, gy = wB * vy, gz = wB * vz;
+                // the large parts of (B_i.r) v_ij and B_i (v_ij.r) cancel here, pair by
+                // pair, before any sum rounds them
+                A.tx.addProduct(msi, fmaT(Bir, vx, -(vr * bi.x)));
+                A.ty.addProduct(msi, fmaT(Bir, vy, -(vr * bi.y)));
+                A.tz.addProduct(msi, fmaT(Bir, vz, -(vr * bi.z)));
                 if(ow.dedner)
                 {
                     // rho_i^2 * m_j (psi_i/rho_i^2 s_i + psi_j/rho_j^2 s_j) r
                     T const g = ow.rho2i * mj * fmaT(bi.w, si, bj.w * sj);
-                    gx = fmaT(g, rx, gx);
-                    gy = fmaT(g, ry, gy);
-                    gz = fmaT(g, rz, gz);
+                    A.tx.addProduct(g, rx);
+                    A.ty.addProduct(g, ry);
+                    A.tz.addProduct(g, rz);
                 }
-                A.tx.add(gx);
-                A.ty.add(gy);
-                A.tz.add(gz);
-                A.divb.add(msi * dBr); // minus m_j s_i (B_i - B_j).r
+                A.divb.addProduct(msi, dBr); // minus m_j s_i (B_i - B_j).r
             }
             A.ax.add(fx);
             A.ay.add(fy);
@@ -488,17 +488,16 @@ namespace sph
             c.d.dudt[t] = pr2 * Dv + A.duav;
             if constexpr(PH >= 2)
             {
-                double const Bi[3] = {c.cur.B[0][t], c.cur.B[1][t], c.cur.B[2][t]};
                 double const psi = c.cur.psi[t];
                 double const* const tv = A.t;
                 double const invRho = 1.0 / rho;
                 double const divB = -invRho * A.divb;
                 double const divv = -invRho * Dv;
                 double const ch = __longlong_as_double(static_cast<long long>(c.bs.chBits[box]));
-                // dB/dt = -(1/rho)(T_induction - B_i D) - rho grad(psi); T carries rho^2 grad(psi)/rho.
+                // dB/dt = -(1/rho) T_induction - rho grad(psi); T carries rho^2 grad(psi)/rho.
 #pragma unroll
                 for(int q = 0; q < 3; ++q)
-                    c.d.dBdt[q][t] = -invRho * (tv[q] - Bi[q] * Dv);
+                    c.d.dBdt[q][t] = -invRho * tv[q];
                 c.d.divB[t] = divB;
                 c.d.dpsidt[t] = dedner ? (-ch * ch * divB - psi * pa.sigma * ch / h - 0.5 * psi * divv) : 0.0;
             }
