@@ -655,9 +655,10 @@ def run_ours(args, rank, world):
         # DRAM bytes per launch from the committed capture, for its own configuration only
         return traffic_from_profiles(name) if profiled_config(args) else None
 
-    # Roofline of the dominant kernel (the longer of the two pair kernels; both
-    # are FP32-pipe / issue bound).  Algorithmic flops count accepted pairs only;
-    # the density kernel's cull of rejected candidates is reported beside it.
+    # Roofline of the dominant pair stage: the density stage (neighbour build and
+    # density sum, two kernels) or the force kernel.  Algorithmic flops count
+    # accepted pairs only; the build's cull of rejected candidates is reported
+    # beside it.
     pairs_step = r["pairs"] / args.steps
     cand_step = r["candidates"]
     force_ms = tm[2] / args.steps
@@ -676,7 +677,7 @@ def run_ours(args, rank, world):
     force_info = {"kernel": f"kForce<{wl_kernel},float,{wl_phys}>", "ms_per_launch": force_ms,
                   "achieved": force_achieved, "frac": force_achieved / peak.value if peak.value else None,
                   "flops_per_pair": flops.FORCE_FLOPS[wl_phys], "traffic": profiled(prof[1])}
-    dens_info = {"kernel": f"kDensity<{wl_kernel},float>", "ms_per_launch": dens_ms,
+    dens_info = {"kernel": f"kNeighbours<float> + kDensity<{wl_kernel},float>", "ms_per_launch": dens_ms,
                  "achieved": dens_achieved, "frac": dens_achieved / peak.value if peak.value else None,
                  "flops_per_pair": flops.DENSITY_FLOPS[wl_kernel], "traffic": profiled(prof[0]),
                  "cull": {"candidates_per_launch": cand_step,
