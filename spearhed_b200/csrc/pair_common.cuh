@@ -100,23 +100,6 @@ namespace sph
         return make_float2(z, z);
     }
 
-    // Unfused arithmetic: the reference's CPU evaluation of the pair geometry.
-    __device__ __forceinline__ float mulRn(float a, float b)
-    {
-        return __fmul_rn(a, b);
-    }
-    __device__ __forceinline__ float addRn(float a, float b)
-    {
-        return __fadd_rn(a, b);
-    }
-    __device__ __forceinline__ double mulRn(double a, double b)
-    {
-        return __dmul_rn(a, b);
-    }
-    __device__ __forceinline__ double addRn(double a, double b)
-    {
-        return __dadd_rn(a, b);
-    }
     //! 1/r from r^2.  At r = 0: FP64 zero; FP32 large and finite, where the
     //! callers' products (r = r^2/r, the kernel slope at r = 0) are zero.
     __device__ __forceinline__ float invDistance(float r2)
@@ -143,16 +126,16 @@ namespace sph
     template<int K>
     __device__ __forceinline__ float slopeOverR(float r, float invR, HConst<float> const& c)
     {
-        float const x = r * c.invh;
+        float const x = mulRn(r, c.invh);
         if constexpr(K == SPH_KERNEL_WENDLAND_C2)
         {
-            float const t = fmaxf(1.f - 0.5f * x, 0.f);
+            float const t = fmaxf(fmaT(-0.5f, x, 1.f), 0.f);
             return c.dwnorm * (-5.f * x * t) * (t * t) * invR;
         }
         else if constexpr(K == SPH_KERNEL_CUBIC)
         {
             float const t = fmaxf(2.f - x, 0.f);
-            return c.dwnorm * (x < 1.f ? (2.25f * x - 3.f) * x : -0.75f * t * t) * invR;
+            return c.dwnorm * (x < 1.f ? fmaT(2.25f, x, -3.f) * x : -0.75f * t * t) * invR;
         }
         else
             return gradWScalar<K, float>(r, invR, c);

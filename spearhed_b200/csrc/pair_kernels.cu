@@ -287,7 +287,7 @@ namespace sph
                     T const dy = own.y - pj.y;
                     T const dz = own.z - pj.z;
                     T const r2 = dot3(dx, dy, dz, dx, dy, dz);
-                    rho.add(pj.w * kernelW<K, T>(r2 * invDistance(r2), hk));
+                    rho.addProduct(pj.w, kernelW<K, T>(r2 * invDistance(r2), hk));
                 };
                 uint32_t const n = min(c.lists.rowLen[t], c.lists.cap);
                 uint32_t const* const row = c.lists.list + rowStart<T>(size_t(t), size_t(c.lists.cap));
@@ -405,21 +405,21 @@ namespace sph
             T const vr = dot3(vx, vy, vz, rx, ry, rz);
             T const msi = mj * si;
             // Isotropic pressure gradient (HydroForces.hpp:155-166).
-            T f = -mj * fmaT(ti.y, si, tj.y * sj);
+            T fs = fmaT(ti.y, si, tj.y * sj);
             T const cb = ow.hc + T(0.5) * tj.z; // mean signal speed
             if(ow.av)
             {
                 // branch-free: mu = 0 (no viscosity) for receding pairs
                 T const vn = vr < T(0) ? vr : T(0);
                 T const hb = ow.hh + T(0.5) * vj.w;
-                T const mu = hb * vn * rcpT(r2 + ow.eps * hb * hb);
+                T const mu = hb * vn * rcpT(fmaT(ow.eps * hb, hb, r2));
                 // Pi_ij (s_i + s_j)/2: the halves of the means 1/rho_ij and s_ij cancel
                 T const Pi = mu * fmaT(ow.beta, mu, -ow.alpha * cb) * rcpT(ti.x + tj.x);
-                T const g = mj * Pi * (si + sj);
-                f -= g;
-                A.duav.addProduct(g, vr); // twice the heating
+                T const g = mulRn(Pi, si + sj);
+                fs += g;
+                A.duav.addProduct(mj * g, vr); // twice the heating
             }
-            T fx = f * rx, fy = f * ry, fz = f * rz;
+            T const f = -mj * fs;
             A.D.addProduct(msi, vr);
             T const w = vr * invR;
             T const vs = fmaT(-ow.beta, w < T(0) ? w : T(0), T(2) * cb);
@@ -430,6 +430,7 @@ namespace sph
                 T const Bir = dot3(bi.x, bi.y, bi.z, rx, ry, rz);
                 T const dBr = dot3(dBx, dBy, dBz, rx, ry, rz);
                 T const cj = mj * tj.w * sj * (Bir + dBr);
+                T fx = f * rx, fy = f * ry, fz = f * rz;
                 if(ow.tensile)
                 {
                     // stress + Borve: c_i B_i + c_j B_j - B_i (c_i + c_j) = c_j (B_j - B_i)
@@ -444,6 +445,9 @@ namespace sph
                     fy = fmaT(cj, bj.y, fmaT(ci, bi.y, fy));
                     fz = fmaT(cj, bj.z, fmaT(ci, bi.z, fz));
                 }
+                A.ax.add(fx);
+                A.ay.add(fy);
+                A.az.add(fz);
                 // the large parts of (B_i.r) v_ij and B_i (v_ij.r) cancel here, pair by
                 // pair, before any sum rounds them
                 A.tx.addProduct(msi, fmaT(Bir, vx, -(vr * bi.x)));
@@ -459,9 +463,12 @@ namespace sph
                 }
                 A.divb.addProduct(msi, dBr); // minus m_j s_i (B_i - B_j).r
             }
-            A.ax.add(fx);
-            A.ay.add(fy);
-            A.az.add(fz);
+            else
+            {
+                A.ax.addProduct(f, rx);
+                A.ay.addProduct(f, ry);
+                A.az.addProduct(f, rz);
+            }
         }
 
         //! The sums of one target, in FP64.

@@ -100,9 +100,28 @@ namespace sph
     }
     constexpr uint32_t kMaxParticles = 1u << 27;
 
-    //! a b + c, rounded once.  Sums of two products are written with it: the
-    //! compiler would fuse one of the two, which one varying from one copy of the
-    //! code to the next, and with it the last bit.
+    // Unfused arithmetic: the reference's CPU evaluation of the pair geometry.
+    __device__ __forceinline__ float mulRn(float a, float b)
+    {
+        return __fmul_rn(a, b);
+    }
+    __device__ __forceinline__ float addRn(float a, float b)
+    {
+        return __fadd_rn(a, b);
+    }
+    __device__ __forceinline__ double mulRn(double a, double b)
+    {
+        return __dmul_rn(a, b);
+    }
+    __device__ __forceinline__ double addRn(double a, double b)
+    {
+        return __dadd_rn(a, b);
+    }
+
+    //! a b + c, rounded once.  Every sum with products in the pair terms is written
+    //! with it (and products that must stay rounded with mulRn): left to the
+    //! compiler, which product it fuses varies from one copy of the code to the
+    //! next, and with it the last bit.
     __device__ __forceinline__ float fmaT(float a, float b, float c)
     {
         return __fmaf_rn(a, b, c);
@@ -141,7 +160,7 @@ namespace sph
         __device__ __forceinline__ static T shapeW(T x)
         {
             if(x < T(1))
-                return T(1) - T(1.5) * x * x + T(0.75) * x * x * x;
+                return fmaT(T(0.75) * x * x, x, fmaT(T(-1.5) * x, x, T(1)));
             if(x < T(2))
             {
                 T const t = T(2) - x;
@@ -154,7 +173,7 @@ namespace sph
         __device__ __forceinline__ static T shapeDW(T x)
         {
             if(x < T(1))
-                return (T(2.25) * x - T(3)) * x;
+                return fmaT(T(2.25), x, T(-3)) * x;
             if(x < T(2))
             {
                 T const t = T(2) - x;
@@ -215,9 +234,9 @@ namespace sph
         {
             if(x < T(2))
             {
-                T const t = T(1) - T(0.5) * x;
+                T const t = fmaT(T(-0.5), x, T(1));
                 T const t2 = t * t;
-                return t2 * t2 * (T(1) + T(2) * x);
+                return t2 * t2 * fmaT(T(2), x, T(1));
             }
             return T(0);
         }
@@ -227,7 +246,7 @@ namespace sph
         {
             if(x < T(2))
             {
-                T const t = T(1) - T(0.5) * x;
+                T const t = fmaT(T(-0.5), x, T(1));
                 return T(-5) * x * t * t * t;
             }
             return T(0);
@@ -257,7 +276,7 @@ namespace sph
     template<int K, typename T>
     __device__ __forceinline__ T kernelW(T r, HConst<T> const& c)
     {
-        return c.wnorm * Kern<K>::shapeW(r * c.invh);
+        return c.wnorm * Kern<K>::shapeW(mulRn(r, c.invh));
     }
 
     //! gradWScalar(r, invR, h) = dW/dr(r, h) * invR: zero when r is not > 0 or
@@ -265,7 +284,7 @@ namespace sph
     template<int K, typename T>
     __device__ __forceinline__ T gradWScalar(T r, T invR, HConst<T> const& c)
     {
-        T const x = r * c.invh;
+        T const x = mulRn(r, c.invh);
         if(!(r > T(0)) || x >= T(Kern<K>::support))
             return T(0);
         return c.dwnorm * Kern<K>::shapeDW(x) * invR;

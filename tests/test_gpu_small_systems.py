@@ -20,19 +20,21 @@ def _run(w, steps=3):
         return ctx.get_species(abi.SPECIES_DEFAULT)
 
 
-@pytest.mark.parametrize("physics", ["mhd", "hydro_av"])
-def test_a_small_box_gets_the_bits_of_the_large_ensemble(physics):
+@pytest.mark.parametrize("physics,kernel", [("mhd", abi.KERNEL_CUBIC), ("mhd", abi.KERNEL_WENDLAND_C2),
+                                            ("mhd", abi.KERNEL_QUINTIC), ("hydro_av", abi.KERNEL_CUBIC)])
+def test_a_small_box_gets_the_bits_of_the_large_ensemble(physics, kernel):
     kw = dict(nbox=8, n_lo=4096, n_hi=16384)
     every = setups.brio_wu_ensemble(**kw)
     n = np.bincount(every.species[abi.SPECIES_DEFAULT].box_id)
     assert n.sum() > 37888 and n.min() <= 9472
     if physics == "hydro_av":
         every.params.physics &= ~(abi.PHYS_MHD | abi.PHYS_DEDNER | abi.PHYS_TENSILE)
+    every.params.kernel = kernel
     whole = _run(every)
     of_box = every.species[abi.SPECIES_DEFAULT].box_id
     for b in (int(np.argmin(n)), int(np.argsort(n)[len(n) // 2])):
         alone = setups.brio_wu_ensemble(**kw, boxes=[b])
-        alone.params.physics = every.params.physics
+        alone.params.physics, alone.params.kernel = every.params.physics, kernel
         got = _run(alone)
         for f in FIELDS:
             assert np.array_equal(getattr(got, f), getattr(whole, f)[..., of_box == b]), (b, f)
