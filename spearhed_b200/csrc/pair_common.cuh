@@ -36,19 +36,6 @@ namespace sph
         return c.r64;
     }
 
-    template<typename T>
-    __device__ __forceinline__ typename PairCfg<T>::V4 const* shiftTable(DevCtx const& c, int box);
-    template<>
-    __device__ __forceinline__ float4 const* shiftTable<float>(DevCtx const& c, int box)
-    {
-        return c.shift32 + size_t(box) * 32;
-    }
-    template<>
-    __device__ __forceinline__ D4 const* shiftTable<double>(DevCtx const& c, int box)
-    {
-        return c.shift64 + size_t(box) * 32;
-    }
-
     //! Paired FP32 arithmetic (sm_100 f32x2) that rounds like the reference's
     //! unfused scalar x, y, z sum.  A paired multiply feeding a paired add is
     //! contracted into a fused multiply-add even when both are written in

@@ -194,7 +194,7 @@ namespace sph
         struct ImageShift<double>
         {
             D4 const* table;
-            __device__ __forceinline__ ImageShift(DevCtx const& c, int box) : table(shiftTable<double>(c, box))
+            __device__ __forceinline__ ImageShift(DevCtx const& c, int box) : table(c.shift64 + size_t(box) * 32)
             {
             }
             __device__ __forceinline__ D4 at(D4 p, uint32_t entry) const

@@ -624,16 +624,13 @@ namespace sph
                 c.bs.hminBits[b] = ~0ull;
             }
             __syncthreads();
-            // stencil shift tables, one entry per thread
+            // stencil shift table, one entry per thread
             for(uint32_t i = threadIdx.x; i < c.nbox * 32u; i += blockDim.x)
             {
                 BoxDev const& B = c.boxes[i >> 5];
                 int const sl = int(i & 31u);
                 bool const used = sl < 27;
                 int const o[3] = {stencilOff(sl, 0), stencilOff(sl, 1), stencilOff(sl, 2)};
-                c.shift32[i] = used ? make_float4(
-                                          float(o[0]) * B.edgef[0], float(o[1]) * B.edgef[1], float(o[2]) * B.edgef[2], 0.f)
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
                 c.shift64[i] = used ? D4{double(o[0]) * B.edge[0], double(o[1]) * B.edge[1], double(o[2]) * B.edge[2], 0.0}
                                     : D4{0.0, 0.0, 0.0, 0.0};
             }
