@@ -652,6 +652,9 @@ namespace sph
                         __syncwarp();
                         sSelf[lane] = ~0u;
                         sSelf[lane + 32] = ~0u;
+                        // another lane may write the same word while staging; the
+                        // shuffles and ballots in between do not order memory
+                        __syncwarp();
                         while(mW + 32u * KB <= uint32_t(CAP))
                         {
                             if(cb >= total)
