@@ -37,6 +37,7 @@
 // for its own work on `stream` before it returns.
 #include "pair_common.cuh"
 
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -181,8 +182,9 @@ namespace
     //!
     //! The acceptance rule is the list-based path's (unfused r^2 in x, y, z order
     //! against R^2); the target itself is its candidate at r = 0, which gives the
-    //! self term.  FP32 lanes fold blocks of 8 candidates by TwoSum; lane sums are
-    //! added in FP64.  rho is written in input order.
+    //! self term (added by hand where R^2 underflows to zero).  FP32 lanes fold
+    //! blocks of 8 candidates by TwoSum; lane sums are added in FP64.  rho is
+    //! written in input order.
     constexpr int kWindow = 128; //!< staged candidates per warp
 
     template<typename T>
@@ -288,10 +290,17 @@ namespace
                     bHi[a] = sph::warpMaxT(act ? x[a] : T(-1e30f));
                 }
                 // rounding is monotone, so with the radius widened by 2^-10 the box
-                // test passes every candidate that the exact test accepts
-                T const reach = R2g * (T(1) + T(1.0 / 1024.0));
+                // test passes every candidate that the exact test accepts; the added
+                // smallest normal number keeps that so where R^2 is denormal and the
+                // factor rounds away
+                constexpr T tiny = sizeof(T) == 4 ? T(FLT_MIN) : T(DBL_MIN);
+                T const reach = R2g * (T(1) + T(1.0 / 1024.0)) + tiny;
                 sph::HConst<T> const hk = sph::hconst<K, T>(hi);
                 sph::Acc<T> rho;
+                // R^2 rounds to zero: no pair is in reach, and the target's own
+                // candidate (r^2 = 0) is not below it either
+                if(R2g == T(0) && act && sub == 0)
+                    rho.add(own.w * sph::kernelW<K, T>(T(0), hk));
                 uint32_t next = 0; // stencil position to stage
                 while(next < total)
                 {
