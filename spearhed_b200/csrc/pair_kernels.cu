@@ -661,12 +661,16 @@ namespace sph
             {
                 // variant 0: SPMHD 4 blocks/SM (128 registers), hydro 5; variant 1 the other
                 constexpr int a = PH >= 2 ? 4 : 5, b = PH >= 2 ? 5 : 4;
-                if(c.n <= (PH >= 2 ? kWideMhd : kWideHydro))
-                    kForce<K, T, PH, a, true><<<rowBlocks(c, kWide), kThreads, 0, s>>>(c, pa);
+                unsigned const wide = rowBlocks(c, kWide), narrow = rowBlocks(c, kLanes<T>);
+                bool const small = c.n <= (PH >= 2 ? kWideMhd : kWideHydro);
+                if(small && variant == 1)
+                    kForce<K, T, PH, b, true><<<wide, kThreads, 0, s>>>(c, pa);
+                else if(small)
+                    kForce<K, T, PH, a, true><<<wide, kThreads, 0, s>>>(c, pa);
                 else if(variant == 1)
-                    kForce<K, T, PH, b><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
+                    kForce<K, T, PH, b><<<narrow, kThreads, 0, s>>>(c, pa);
                 else
-                    kForce<K, T, PH, a><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
+                    kForce<K, T, PH, a><<<narrow, kThreads, 0, s>>>(c, pa);
             }
             else
                 kForce<K, T, PH, 3><<<rowBlocks(c, kLanes<T>), kThreads, 0, s>>>(c, pa);
@@ -731,7 +735,8 @@ namespace sph
         template<int K, int PH>
         void configureForceK()
         {
-            preferL1(kForce<K, float, PH, PH >= 2 ? 4 : 5, true>);
+            preferL1(kForce<K, float, PH, 4, true>);
+            preferL1(kForce<K, float, PH, 5, true>);
             preferL1(kForce<K, float, PH, 4>);
             preferL1(kForce<K, float, PH, 5>);
             preferL1(kForce<K, double, PH, 3>);

@@ -37,6 +37,12 @@ SHAPE_CASES = {
 }
 
 
+# Above the particle counts up to which the FP32 force pass gives a row eight lanes
+# (9,472 with MHD, 18,944 without): the one-lane kernels' shapes.
+SHAPE_CASES["orszag_tang_one_lane"] = lambda prec: setups.orszag_tang(nx=50, nz=4, precision=prec, jitter=0.1)
+SHAPE_CASES["sod_one_lane"] = lambda prec: setups.sod_small(precision=prec, scale=1.25)
+
+
 @pytest.mark.parametrize("prec", [abi.PREC_FP32_COMP, abi.PREC_FP64])
 @pytest.mark.parametrize("case", list(SHAPE_CASES))
 def test_every_shape_gives_the_same_bits(prec, case):
@@ -80,3 +86,35 @@ def test_autotune_keeps_the_state():
     ctx.step(1)
     assert ctx.reduce()["steps"] == 3
     ctx.close()
+
+
+@pytest.mark.parametrize("case", ["orszag_tang", "orszag_tang_one_lane", "sod", "sod_one_lane"])
+def test_each_force_variant_is_a_kernel_of_its_own(case):
+    """The shape that sph_set_tuning asks for is the one that runs, in small
+    systems (eight lanes per row) as in large ones: the launched kernel's
+    blocks-per-SM argument is what sph_get_tuning reports."""
+    import re
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    import spearhed_b200 as sb
+    make = SHAPE_CASES.get(case, lambda prec: setups.sod_small(precision=prec, scale=0.5))
+    w = make(abi.PREC_FP32_COMP)
+    with sb.context_for(w) as ctx:
+        shapes = []
+        for fv in range(ctx.tuning()["n_force_variants"]):
+            ctx.set_tuning(0, fv)
+            ctx.step(1)
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                ctx.step(1)
+                torch.cuda.synchronize()
+            traced = [e.key for e in prof.key_averages()]
+            if not traced:
+                pytest.skip("the profiler records no kernels here")
+            names = {k for k in traced if "kForce" in k}
+            assert len(names) == 1, names
+            # kForce<kernel, precision, physics, blocks per SM, eight lanes>
+            args = re.search(r"kForce<([^>]*)>", names.pop()).group(1).split(", ")
+            assert args[4] == ("false" if case.endswith("one_lane") else "true")
+            assert int(args[3]) == ctx.tuning()["force_blocks_per_sm"], (fv, args)
+            shapes.append(args[3])
+        assert len(set(shapes)) == len(shapes) == 2, shapes
