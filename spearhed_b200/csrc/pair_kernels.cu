@@ -415,7 +415,7 @@ namespace sph
                 T const mu = hb * vn * rcpT(fmaT(ow.eps * hb, hb, r2));
                 // Pi_ij (s_i + s_j)/2: the halves of the means 1/rho_ij and s_ij cancel
                 T const Pi = mu * fmaT(ow.beta, mu, -ow.alpha * cb) * rcpT(ti.x + tj.x);
-                T const g = mulRn(Pi, si + sj);
+                T const g = mulRn(Pi, addRn(si, sj));
                 fs += g;
                 A.duav.addProduct(mj * g, vr); // twice the heating
             }
@@ -477,7 +477,8 @@ namespace sph
             double a[3], D, duav, t[3], divb, vsig;
         };
 
-        //! FP64 epilogue of one target: derivatives and its CFL time step.
+        //! FP64 epilogue of one target: derivatives and its CFL time step.  Roundings are
+        //! spelled out (see fmaT): the one-lane and the eight-lane kernel each hold a copy.
         template<int PH>
         __device__ __forceinline__ double forceEpilogue(
             DevCtx const& c,
@@ -492,7 +493,7 @@ namespace sph
             double const pr2 = (pa.gamma - 1.0) * c.cur.u[t] / rho; // P_i / rho_i^2
             double const* const a = A.a;
             double const Dv = A.D;
-            c.d.dudt[t] = pr2 * Dv + A.duav;
+            c.d.dudt[t] = fmaT(pr2, Dv, A.duav);
             if constexpr(PH >= 2)
             {
                 double const psi = c.cur.psi[t];
@@ -506,13 +507,14 @@ namespace sph
                 for(int q = 0; q < 3; ++q)
                     c.d.dBdt[q][t] = -invRho * tv[q];
                 c.d.divB[t] = divB;
-                c.d.dpsidt[t] = dedner ? (-ch * ch * divB - psi * pa.sigma * ch / h - 0.5 * psi * divv) : 0.0;
+                double const decay = psi * pa.sigma * ch / h;
+                c.d.dpsidt[t] = dedner ? fmaT(-0.5 * psi, divv, fmaT(-ch * ch, divB, -decay)) : 0.0;
             }
 #pragma unroll
             for(int q = 0; q < 3; ++q)
                 c.d.dvdt[q][t] = a[q];
             double dt = pa.cfl * h / A.vsig;
-            double const amag = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
+            double const amag = sqrt(dot3(a[0], a[1], a[2], a[0], a[1], a[2]));
             if(amag > 0.0 && pa.cflForce > 0.0)
                 dt = fmin(dt, pa.cflForce * sqrt(h / amag));
             return dt;

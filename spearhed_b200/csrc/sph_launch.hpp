@@ -67,6 +67,8 @@ namespace sph
     //! Derived per-particle quantities the force pass reads for a source:
     //! ft = (rho, (P + B^2/(2 mu0))/rho^2, c, 1/(mu0 rho^2)), fb = (B, psi/rho^2).
     //! c is the sound speed, or the fast speed sqrt(c_s^2 + B^2/(mu0 rho)) with MHD.
+    //! Roundings are spelled out (see fmaT): two density kernels and the permute
+    //! compute the same records.
     __device__ __forceinline__ void derivedRecord(
         double rho,
         double u,
@@ -77,12 +79,12 @@ namespace sph
         double fb[4])
     {
         bool const mhd = pa.physics & SPH_PHYS_MHD;
-        double const P = (pa.gamma - 1.0) * rho * u;
+        double const P = mulRn((pa.gamma - 1.0) * rho, u);
         double const inv2 = 1.0 / (rho * rho);
         double const cs2 = pa.gamma * P / rho;
         double B2 = 0.0;
         if(mhd)
-            B2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
+            B2 = dot3(B[0], B[1], B[2], B[0], B[1], B[2]);
         ft[0] = rho;
         ft[1] = (P + (mhd ? 0.5 * B2 / pa.mu0 : 0.0)) * inv2;
         ft[2] = sqrt(cs2 + (mhd ? B2 / (pa.mu0 * rho) : 0.0));
