@@ -227,18 +227,24 @@ namespace sph
         //! accepts it; up = 31 - lane.  The mask's bits up to the lane's own are
         //! moved to the top: the sign is its own bit, the population its place.
         //! The store is predicated (a branch around it would add the warp's
-        //! divergence bookkeeping to every target).
+        //! divergence bookkeeping to every target).  room: words of the lists from
+        //! rows on (bounds-checked builds).
         template<typename T>
         __device__ __forceinline__ void storeEntry(
             typename RowRef<T>::Type r,
             uint32_t up,
             uint32_t* rows,
-            uint32_t ent)
+            uint32_t ent,
+            size_t room,
+            uint32_t* status)
         {
             uint32_t const b = r.x << up;
+            uint32_t const place = RowRef<T>::place(r, uint32_t(__popc(b)));
+            if(!checkIndex(int32_t(b) >= 0 || place < room, status, kChkRowStore))
+                return;
             asm volatile("{ .reg .pred q; setp.lt.s32 q, %0, 0; @q st.global.u32 [%1], %2; }"
                          :
-                         : "r"(b), "l"(rows + RowRef<T>::place(r, uint32_t(__popc(b)))), "r"(ent)
+                         : "r"(b), "l"(rows + place), "r"(ent)
                          : "memory");
         }
 
@@ -274,6 +280,8 @@ namespace sph
             T supT,
             T R2g,
             uint32_t* rows,
+            size_t room,
+            uint32_t* status,
             uint32_t cap,
             int lane,
             bool countOnly)
@@ -328,7 +336,7 @@ namespace sph
                     for(uint32_t i = 0; i < nt; i += 8)
 #pragma unroll
                         for(uint32_t u = 0; u < 8; ++u)
-                            storeEntry<T>(sRow[i + u], up, rows, ent);
+                            storeEntry<T>(sRow[i + u], up, rows, ent, room, status);
                     continue;
                 }
                 int const nS = int(min(uint32_t(S), nSlab - g0));
@@ -337,7 +345,7 @@ namespace sph
                     uint32_t const ent = sEnt[((g0 + uint32_t(s)) << 5) + uint32_t(lane)];
 #pragma unroll 4
                     for(uint32_t i = 0; i < nt; ++i)
-                        storeEntry<T>(sRow[i * uint32_t(S) + uint32_t(s)], up, rows, ent);
+                        storeEntry<T>(sRow[i * uint32_t(S) + uint32_t(s)], up, rows, ent, room, status);
                 }
             }
         }
@@ -756,9 +764,10 @@ namespace sph
                         {
                             TargetChunk<T> ch = w ? Bc : A;
                             uint32_t const first = tc + 32u * uint32_t(w);
+                            size_t const row0 = rowStart<T>(size_t(first & ~3u), size_t(cap));
                             cullChunk<T, PAIRMAX, CU>(
                                 ch, sNX, sNY, sNZ, sH, sEnt, sSelf + 32 * w, sRow, first, w ? ntB : ntA, m, supT, R2g,
-                                c.lists.list + rowStart<T>(size_t(first & ~3u), size_t(cap)), cap, lane, countOnly);
+                                c.lists.list + row0, listWords(c.n, cap) - row0, c.status, cap, lane, countOnly);
                             if(w)
                                 Bc = ch;
                             else

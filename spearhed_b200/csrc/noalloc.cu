@@ -55,6 +55,7 @@ namespace
     constexpr uint32_t kMaxParticles = 1u << 18;
     constexpr uint32_t kMaxCells = 1u << 18;
     constexpr int kMaxDevices = 64;
+    constexpr int kStatus = sph::kStatWords; //!< status words of a call; the bounds checks set kStatCheck
 
     static __device__ __align__(256) unsigned char g_noallocScratch[kScratchBytes];
 
@@ -143,6 +144,7 @@ namespace
     __global__ void kPackSorted(
         sph::BoxDev const B,
         uint32_t n,
+        uint32_t* status,
         uint32_t const* __restrict__ perm,
         double const* __restrict__ x,
         double const* __restrict__ y,
@@ -156,6 +158,8 @@ namespace
         if(p >= n)
             return;
         uint32_t const q = perm[p];
+        if(!sph::checkIndex(q < n, status, sph::kChkPermute))
+            return;
         double const pos[3] = {x[q], y[q], z[q]};
         double rel[3];
         for(int a = 0; a < 3; ++a)
@@ -206,6 +210,8 @@ namespace
     template<int K, typename V4, typename T>
     __global__ void __launch_bounds__(kWarps * 32) kDensityStaged(
         sph::BoxDev const box,
+        uint32_t n,
+        uint32_t* status,
         sph::Cells cells,
         uint32_t const* __restrict__ perm,
         V4 const* __restrict__ pm,
@@ -223,7 +229,7 @@ namespace
         {
             uint32_t const cell = q >> partShift;
             uint32_t const tBeg = cells.start[cell] + (q & ((1u << partShift) - 1u)) * group, tEnd = cells.mid[cell];
-            if(tBeg >= tEnd)
+            if(tBeg >= tEnd || !sph::checkIndex(tEnd <= n, status, sph::kChkTargets))
                 continue;
             // lane d < 27: the source range and image shift of stencil slot d
             uint32_t sBeg = 0, cnt = 0;
@@ -251,8 +257,13 @@ namespace
                 if(ok)
                 {
                     uint32_t const ncell = (uint32_t(nc[2]) * n1 + uint32_t(nc[1])) * n0 + uint32_t(nc[0]);
-                    sBeg = cells.start[ncell];
-                    cnt = cells.end[ncell] - sBeg;
+                    if(sph::checkIndex(ncell < cells.ncells, status, sph::kChkCell))
+                    {
+                        sBeg = cells.start[ncell];
+                        cnt = cells.end[ncell] - sBeg;
+                    }
+                    if(!sph::checkIndex(sBeg <= n && cnt <= n - sBeg, status, sph::kChkRange))
+                        cnt = 0;
                 }
             }
             uint32_t pre = cnt;
@@ -320,7 +331,7 @@ namespace
                                 sz = __shfl_sync(0xffffffffu, sh[2], d);
                         bool pass = false;
                         V4 c{};
-                        if(p < total)
+                        if(p < total && sph::checkIndex(j < n, status, sph::kChkStaged))
                         {
                             c = sph::ld4(pm + j);
                             c.x = -sph::addRn(c.x, sx);
@@ -331,8 +342,9 @@ namespace
                             pass = dx * dx + dy * dy + dz * dz < reach;
                         }
                         uint32_t const passed = __ballot_sync(0xffffffffu, pass);
-                        if(pass)
-                            win[m + uint32_t(__popc(passed & ((1u << lane) - 1u)))] = c;
+                        uint32_t const w = m + uint32_t(__popc(passed & ((1u << lane) - 1u)));
+                        if(pass && sph::checkIndex(w < uint32_t(kWindow), status, sph::kChkWindow))
+                            win[w] = c;
                         m += uint32_t(__popc(passed));
                         next += 32;
                     }
@@ -356,7 +368,11 @@ namespace
                 for(int o = 1; o < S; o <<= 1)
                     v += __shfl_xor_sync(0xffffffffu, v, o);
                 if(act && sub == 0)
-                    rhoOut[perm[t]] = v;
+                {
+                    uint32_t const q = perm[t];
+                    if(sph::checkIndex(q < n, status, sph::kChkPermute))
+                        rhoOut[q] = v;
+                }
             }
         }
     }
@@ -365,6 +381,7 @@ namespace
     void launchStaged(
         sph::BoxDev const& box,
         uint32_t n,
+        uint32_t* status,
         sph::Cells const& cells,
         uint32_t const* perm,
         V4 const* pm,
@@ -387,7 +404,7 @@ namespace
         // the global cull radius only: pair-max calls are refused before any launch
         T const Rg = T(sph::Kern<K>::support) * T(p.h0);
         kDensityStaged<K, V4, T>
-            <<<blocks, kWarps * 32, 0, s>>>(box, cells, perm, pm, hc, T(Rg * Rg), group, partShift, rho);
+            <<<blocks, kWarps * 32, 0, s>>>(box, n, status, cells, perm, pm, hc, T(Rg * Rg), group, partShift, rho);
         sph::countLaunches(1);
     }
 
@@ -395,6 +412,7 @@ namespace
     void launchStagedK(
         sph::BoxDev const& box,
         uint32_t n,
+        uint32_t* status,
         sph::Cells const& cells,
         uint32_t const* perm,
         V4 const* pm,
@@ -404,11 +422,11 @@ namespace
         cudaStream_t s)
     {
         if(p.kernel == SPH_KERNEL_QUINTIC)
-            launchStaged<SPH_KERNEL_QUINTIC>(box, n, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_QUINTIC>(box, n, status, cells, perm, pm, hc, p, rho, s);
         else if(p.kernel == SPH_KERNEL_WENDLAND_C2)
-            launchStaged<SPH_KERNEL_WENDLAND_C2>(box, n, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_WENDLAND_C2>(box, n, status, cells, perm, pm, hc, p, rho, s);
         else
-            launchStaged<SPH_KERNEL_CUBIC>(box, n, cells, perm, pm, hc, p, rho, s);
+            launchStaged<SPH_KERNEL_CUBIC>(box, n, status, cells, perm, pm, hc, p, rho, s);
     }
 } // namespace
 
@@ -483,7 +501,7 @@ int sph_density_noalloc(
     uint32_t const nn = uint32_t(n);
     bool const fp64 = p.precision == SPH_PREC_FP64;
     Carve cv{static_cast<unsigned char*>(base)};
-    uint32_t* status = cv.take<uint32_t>(4);
+    uint32_t* status = cv.take<uint32_t>(kStatus);
     uint32_t* keysA = cv.take<uint32_t>(nn);
     uint32_t* valsA = cv.take<uint32_t>(nn);
     uint32_t* keysB = cv.take<uint32_t>(nn);
@@ -519,7 +537,7 @@ int sph_density_noalloc(
     (void)cudaGetLastError();
     // Everything below is stream-ordered; nothing that must start at zero is
     // assumed to be zero from an earlier call.
-    if(cudaMemsetAsync(status, 0, 4 * sizeof(uint32_t), s) != cudaSuccess)
+    if(cudaMemsetAsync(status, 0, kStatus * sizeof(uint32_t), s) != cudaSuccess)
         return failNoAlloc(SPH_ERR_CUDA, "sph_density_noalloc: stream operation failed");
     auto launched = [](char const* what) -> int
     {
@@ -550,25 +568,25 @@ int sph_density_noalloc(
         return st;
     if(fp64)
     {
-        kPackSorted<sph::D4, double><<<g, kThreads, 0, s>>>(bd, nn, perm, x, y, z, mass, h, pm64, hc64);
+        kPackSorted<sph::D4, double><<<g, kThreads, 0, s>>>(bd, nn, status, perm, x, y, z, mass, h, pm64, hc64);
         sph::countLaunches(1);
         if((st = launched("packing")))
             return st;
-        launchStagedK<sph::D4, double>(bd, nn, cells, perm, pm64, hc64, p, rho, s);
+        launchStagedK<sph::D4, double>(bd, nn, status, cells, perm, pm64, hc64, p, rho, s);
     }
     else
     {
-        kPackSorted<float4, float><<<g, kThreads, 0, s>>>(bd, nn, perm, x, y, z, mass, h, pm32, hc32);
+        kPackSorted<float4, float><<<g, kThreads, 0, s>>>(bd, nn, status, perm, x, y, z, mass, h, pm32, hc32);
         sph::countLaunches(1);
         if((st = launched("packing")))
             return st;
-        launchStagedK<float4, float>(bd, nn, cells, perm, pm32, hc32, p, rho, s);
+        launchStagedK<float4, float>(bd, nn, status, cells, perm, pm32, hc32, p, rho, s);
     }
     if((st = launched("density")))
         return st;
     // Bad inputs are only known after the work ran, so the density kernel is
     // told nothing; rho is written but must not be used on an error return.
-    uint32_t bad[2] = {0, 0};
+    uint32_t bad[kStatus] = {};
     cudaError_t e = cudaMemcpyAsync(bad, status, sizeof(bad), cudaMemcpyDeviceToHost, s);
     if(e == cudaSuccess)
         e = cudaStreamSynchronize(s);
@@ -582,6 +600,11 @@ int sph_density_noalloc(
     if(bad[0])
         return failNoAlloc(
             SPH_ERR_OUTSIDE, "sph_density_noalloc: " + std::to_string(bad[0]) + " particles outside the box");
+    if(bad[sph::kStatCheck])
+        return failNoAlloc(
+            SPH_ERR_STATE,
+            "sph_density_noalloc: a device bounds check failed (sites " + std::to_string(bad[sph::kStatCheck])
+                + "; the access was skipped and rho is not valid)");
     return SPH_OK;
 }
 }

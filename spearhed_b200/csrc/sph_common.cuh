@@ -344,8 +344,9 @@ namespace sph
         kChkTargets = 3,    //!< a target cell's range within the particles
         kChkRowEntry = 4,   //!< a list entry read back (particle index and stencil slot)
         kChkPermute = 5,    //!< a permutation index
-        kChkKey = 6,        //!< a sorted cell key within the cells
-        kChkDriftCell = 7   //!< a particle's cell id from the drift
+        kChkDriftCell = 7,  //!< a particle's cell id from the drift
+        kChkRowStore = 8,   //!< a list entry's place as it is written
+        kChkWindow = 9      //!< a staging window's position (allocation-free density)
     };
 
     //! Bounds-checked builds (compiled with -DSPH_CHECK): a failed check sets

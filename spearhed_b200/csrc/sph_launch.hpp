@@ -193,7 +193,7 @@ namespace sph
             return k;
     }
     //! Words of the lists of n targets.
-    inline size_t listWords(size_t n, size_t cap)
+    __host__ __device__ inline size_t listWords(size_t n, size_t cap)
     {
         return ((n + 3) & ~size_t(3)) * cap;
     }

@@ -2,16 +2,16 @@
 -DSPH_CHECK).
 
 Its kernels check the indices they read through (stencil cell ids, cell
-source ranges, staged candidates, target ranges, list entries read back,
-permutation indices, sorted cell keys, drift cells) and, on a failed check,
-set that site's bit in a status word and skip the access; the host turns the
-word into SPH_ERR_STATE.  It is the substitute for compute-sanitizer, which is
-closed on this pool.
+source ranges, staged candidates, target ranges, list entries as they are
+written and read back, permutation indices, drift cells, the allocation-free
+density's windows) and, on a failed check, set that site's bit in a status word
+and skip the access; the host turns the word into SPH_ERR_STATE.
 
 Without a GPU: the checked library loads and exports every declared entry
-point.  With one: the parity, ensemble, species and configuration tests run
-on the checked library (a child pytest with SPEARHED_B200_VARIANT=check) and
-pass, i.e. no check fires and every result still matches the oracle.
+point.  With one: the parity, ensemble, species and configuration tests and
+those of the size-dependent paths run on the checked library (a child pytest
+with SPEARHED_B200_VARIANT=check) and pass, i.e. no check fires and every
+result still matches the oracle.
 """
 import os
 import re
@@ -49,7 +49,8 @@ def test_checked_library_loads_and_exports_the_boundary():
 @pytest.mark.gpu
 def test_parity_suites_pass_on_the_checked_build():
     files = ["tests/test_gpu_parity.py", "tests/test_gpu_ensemble.py", "tests/test_gpu_species.py",
-             "tests/test_gpu_configs.py"]
+             "tests/test_gpu_configs.py", "tests/test_gpu_target_groups.py", "tests/test_gpu_small_systems.py",
+             "tests/test_gpu_noalloc_groups.py"]
     r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider"] + files,
                        cwd=ROOT, env=_env(), capture_output=True, text=True, timeout=1800)
     tail = "\n".join(r.stdout.splitlines()[-15:])
