@@ -83,9 +83,9 @@ def test_every_pair_in_reach(oracle, prec, cull, n):
     other's reach, the accepted pairs are all n(n-1) ordered pairs, self
     excluded.  n particles in [0.4, 0.6]^3 with h = 0.5 (cull radius 1, above
     the cloud's diameter) in a non-periodic unit box: one cell holds them all,
-    every acceptance mask is full, and the cell runs full chunks plus a short
-    tail chunk (n = 33: one target on 32 sub-lanes; n = 200: eight targets on
-    four).  The densities are the oracle's."""
+    every acceptance mask is full, and the cell's targets are dealt to warps in
+    groups of four on eight sub-lanes each (n = 33: and one target on 32).  The
+    densities are the oracle's."""
     rng = np.random.default_rng(7)
     s = abi.Species(n)
     s.pos[:] = 0.4 + 0.2 * rng.random((3, n))
@@ -200,7 +200,7 @@ def test_pairs_at_the_cull_radius_match_oracle(oracle, kernel, prec):
     cell-relative positions and every distance are exact.  Pairs at r = R and
     beyond are rejected (strict r^2 < R^2) and the 26 offsets with
     i^2 + j^2 + k^2 <= 3 are accepted, through the staging box test, in cells
-    of 8 to 27 targets (short and full chunks)."""
+    of 8 to 27 targets (groups of four, full and part-filled)."""
     dx = 1.0 / 16.0
     g = np.arange(10) * dx
     X, Y, Z = np.meshgrid(g, g, g, indexing="ij")
@@ -232,9 +232,10 @@ def test_pairs_at_the_cull_radius_match_oracle(oracle, kernel, prec):
 @pytest.mark.parametrize("cull,vary", [(abi.CULL_GLOBAL, False), (abi.CULL_PAIR_MAX, True)])
 def test_dense_cluster_matches_oracle(oracle, kernel, prec, cull, vary):
     """A tenth of the box's particles in a ball of radius 0.04 inside a uniform
-    cloud: the cluster's cells hold hundreds of targets, so a cell runs many
-    64-target chunk pairs, each with its own staging box, plus a short tail
-    chunk; the accepted pair sets are the oracle's and the densities agree."""
+    cloud: the cluster's cells hold hundreds of targets, dealt to warps in groups
+    of four (so few particles), each group with its own staging box; the accepted
+    pair sets are the oracle's and the densities agree.  (Dense cells at the
+    particle counts where groups hold 64: test_gpu_target_groups.py.)"""
     p, boxes, sp = _cloud(kernel, prec, n=3000, cull=cull, vary_h=vary)
     s = sp[abi.SPECIES_DEFAULT]
     rng = np.random.default_rng(11)
@@ -270,6 +271,54 @@ def test_hydro_matches_oracle(oracle, kernel, prec, physics):
     orc.force()
     assert _normwise(got.dvdt, orc.s.dvdt) <= TOL[prec]["acc"]
     assert _normwise(got.dudt, orc.s.dudt) <= TOL[prec]["acc"]
+
+
+@pytest.mark.parametrize("kernel", [CUBIC, QUINTIC, WENDLAND])
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("physics", [0, abi.PHYS_AV])
+def test_hydro_above_the_small_system_limit_matches_oracle(oracle, kernel, prec, physics):
+    """As test_hydro_matches_oracle, at a particle count where the FP32 force pass
+    gives a row one lane (up to 18,944 it gives it eight)."""
+    p, boxes, sp = _cloud(kernel, prec, n=20011, physics=physics)
+    ctx = _ctx(p, boxes, sp)
+    ctx.density()
+    ctx.hydro()
+    got = ctx.get_species(abi.SPECIES_DEFAULT)
+    ctx.close()
+    orc = _oracle(oracle, p, boxes, sp)
+    orc.density()
+    orc.force()
+    assert _normwise(got.dvdt, orc.s.dvdt) <= TOL[prec]["acc"]
+    assert _normwise(got.dudt, orc.s.dudt) <= TOL[prec]["acc"]
+
+
+MHD_EXTRAS = abi.PHYS_AV | abi.PHYS_DEDNER | abi.PHYS_TENSILE
+
+
+@pytest.mark.parametrize("kernel", [CUBIC, QUINTIC, WENDLAND])
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("off", [0, abi.PHYS_DEDNER, MHD_EXTRAS])
+@pytest.mark.parametrize("nx", [32, 50])
+def test_mhd_variants_match_oracle(oracle, kernel, prec, off, nx):
+    """SPMHD with all its extras, without Dedner cleaning and without any of them
+    (kernels of their own), on both sides of the particle count (9,472) up to
+    which the FP32 force pass gives a row eight lanes."""
+    w = setups.orszag_tang(nx=nx, nz=5, precision=prec, jitter=0.1)
+    w.params.kernel = kernel
+    w.params.physics &= ~off
+    rng = np.random.default_rng(nx)
+    w.species[abi.SPECIES_DEFAULT].psi[:] = 0.1 * rng.normal(size=nx * nx * 5)
+    ctx = _ctx(w.params, w.boxes, w.species)
+    ctx.density()
+    ctx.mhd()
+    got = ctx.get_species(abi.SPECIES_DEFAULT)
+    ctx.close()
+    orc = _oracle(oracle, w.params, w.boxes, w.species)
+    orc.density()
+    orc.force()
+    for f in ("dvdt", "dudt", "dBdt"):
+        err = _normwise(getattr(got, f), getattr(orc.s, f))
+        assert err <= TOL[prec]["acc"], (f, err)
 
 
 @pytest.mark.parametrize("prec", PRECS)

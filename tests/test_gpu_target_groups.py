@@ -2,8 +2,9 @@
 or 4, by the number of particles.  One slab per group size (for either
 precision; its full and part-filled chunks, odd counts per cell) against the
 oracle: per-particle neighbour counts exact in the precision's geometry, density
-within the parity bounds (FP64 1e-12, FP32 1e-5 relative).  nx = 120 is also a size whose cell sort scans
-its digit rows in a launch of their own; the others let the scatter add them.
+within the parity bounds (FP64 1e-12, FP32 1e-5 relative).  nx = 120, 191 and 269
+are also sizes whose cell sort scans its digit rows in a launch of their own (more
+than 192 tiles); the others let the scatter add them.
 """
 import numpy as np
 import pytest

@@ -26,10 +26,10 @@ def _steps(w, dv, fv, n=3):
     return out
 
 
-# OT: one level, global cull, mostly full chunks.  Rotor and a small Brio-Wu
-# ensemble: two cell levels, the pair-max cull and cells of few targets, so the
-# short chunks' slab cull, the skewed staging slabs and the own-entry positions
-# run in every shape.
+# OT: one level, global cull.  Rotor and a small Brio-Wu ensemble: two cell levels,
+# the pair-max cull and cells of few targets.  At these particle counts a cell's
+# targets are taken in groups of 4 or 8, so the short chunks' slab cull, the skewed
+# staging slabs and the own-entry positions run in every shape.
 SHAPE_CASES = {
     "orszag_tang": lambda prec: setups.orszag_tang(nx=32, nz=4, precision=prec, jitter=0.1),
     "mhd_rotor": lambda prec: setups.mhd_rotor(nxy=64, precision=prec),
@@ -40,6 +40,9 @@ SHAPE_CASES = {
 # Above the particle counts up to which the FP32 force pass gives a row eight lanes
 # (9,472 with MHD, 18,944 without): the one-lane kernels' shapes.
 SHAPE_CASES["orszag_tang_one_lane"] = lambda prec: setups.orszag_tang(nx=50, nz=4, precision=prec, jitter=0.1)
+# Above the particle counts where groups hold 64 targets: full chunks.
+SHAPE_CASES["orszag_tang_full_groups"] = lambda prec: setups.orszag_tang(nx=270, nz=4, precision=prec, jitter=0.1)
+SHAPE_CASES["mhd_rotor_full_groups"] = lambda prec: setups.mhd_rotor(nxy=240, precision=prec)
 SHAPE_CASES["sod_one_lane"] = lambda prec: setups.sod_small(precision=prec, scale=1.25)
 
 
