@@ -354,14 +354,37 @@ namespace sph
         //! warps in groups of 64 >> shift.  A group shares its staged windows, so
         //! large groups cost least work, but few particles in groups of 64 leave
         //! most warps idle behind the cells with the longest stencils: the group
-        //! halves until n / group fills the resident warps 1.25 times.  Density
-        //! pass at groups of 64 / 32 / 16 / 8 / 4, ms: FP64 Sod 2.3 k 0.195 / 0.147 /
-        //! 0.116 / 0.102 / 0.098; FP32 Sod 18 k 0.167 / 0.136 / 0.135 / 0.130 / 0.128;
-        //! FP64 Brio-Wu 176 k 0.349 / 0.316 / 0.337 / 0.426 / 0.639; FP64 Orszag-Tang
-        //! 206 k 0.306 / 0.323 / 0.354 / 0.453 / 0.651; FP32 Brio-Wu 2 M 1.37 / 1.56 /
-        //! 1.82 / 2.60 / 4.35.  Grids with many more cells than particles are not
-        //! split (each part asks for the cell's range).  The rows are the same for
-        //! every group: a target's entries keep their candidate order.
+        //! halves until n / group fills the resident warps 1.25 times (FP32: 64 from
+        //! 284,160 particles on, 32 from 142,080 and so on; FP64: 189,440, 94,720, ...).
+        //! Neighbour build and density sum at groups of 64 / 32 / 16 / 8 / 4, ms, * the
+        //! one this line picks:
+        //!   FP32 Sod         2.3 k  0.085 / 0.057 / 0.049 / 0.045 / 0.049*
+        //!        Sod          18 k  0.109 / 0.082 / 0.086 / 0.086 / 0.084*
+        //!        Orszag-Tang  50 k  0.093 / 0.104 / 0.100 / 0.096* / 0.113
+        //!        Orszag-Tang 100 k  0.144 / 0.134 / 0.132* / 0.143 / 0.177
+        //!        Orszag-Tang 201 k  0.191 / 0.199* / 0.216 / 0.250 / 0.321
+        //!        Orszag-Tang 300 k  0.235* / 0.261 / 0.290 / 0.346 / 0.457
+        //!        Brio-Wu      60 k  0.137 / 0.105 / 0.108 / 0.118* / 0.149
+        //!        Brio-Wu      82 k  0.158 / 0.117 / 0.124* / 0.131 / 0.186
+        //!        Brio-Wu     224 k  0.230 / 0.199* / 0.222 / 0.287 / 0.446
+        //!        Brio-Wu     581 k  0.433* / 0.417 / 0.481 / 0.634 / 1.043
+        //!        Brio-Wu       2 M  1.212* / 1.233 / 1.478 / 2.096 / 3.695
+        //!   FP64 Sod         2.3 k  0.137 / 0.081 / 0.069 / 0.061 / 0.062*
+        //!        Orszag-Tang 100 k  0.186 / 0.179* / 0.189 / 0.219 / 0.287
+        //!        Orszag-Tang 151 k  0.204 / 0.227* / 0.245 / 0.294 / 0.400
+        //!        Orszag-Tang 180 k  0.249 / 0.264* / 0.289 / 0.349 / 0.475
+        //!        Orszag-Tang 201 k  0.264* / 0.285 / 0.312 / 0.382 / 0.521
+        //!        Brio-Wu     109 k  0.260 / 0.198* / 0.201 / 0.241 / 0.356
+        //!        Brio-Wu     176 k  0.316 / 0.246* / 0.266 / 0.361 / 0.550
+        //!        Brio-Wu     224 k  0.364* / 0.296 / 0.346 / 0.465 / 0.729
+        //!        Brio-Wu     263 k  0.399* / 0.343 / 0.390 / 0.510 / 0.811
+        //! The particle count alone is a compromise: one-level slabs want 64 from
+        //! somewhere below 150 k (FP64) or 200 k (FP32) particles on, two-level tubes 32
+        //! up to 263 k and more (FP64) or 581 k (FP32).  At the points above the line
+        //! costs up to 11% on the slabs' side and 23% on the tubes'.
+        //! Grids with many more cells than particles are not split (each part asks for
+        //! the cell's range).  The rows are the same for every group: a target's
+        //! entries keep their candidate order.
         constexpr int kMaxPartShift = 4;
         __device__ __forceinline__ int partsShift(uint32_t n, uint32_t cells, uint32_t warps)
         {
@@ -475,8 +498,9 @@ namespace sph
                 // two or three images.  Such axes run fastest, equal cells adjacent (-1,
                 // +1, 0), so a row lists a cell's images one after another and the lanes
                 // of a pair pass, which stand at different images, stay on the same
-                // lines of records: 16.8 -> 12 lines a request on the Orszag-Tang slab
-                // (one cell thick), force pass 0.643 -> 0.600 ms.
+                // lines of records: 16.8 -> 12.0 distinct lines a request on the
+                // Orszag-Tang slab (one cell thick; simulated), force pass 0.643 -> 0.600
+                // ms when it was made.
                 int const nDesc = 27 + (B.levels == 2 ? 27 : 0);
                 auto describe = [&](int d, uint32_t& sBeg, uint32_t& sCnt, uint32_t& slot, T sh[3])
                 {

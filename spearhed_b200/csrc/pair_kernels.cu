@@ -7,15 +7,19 @@
 // writes rho (FP64) and the target's derived record for the force pass.
 //
 // What bounds both passes is the gather of the sources' 16-byte records: a warp
-// request costs the L1 one wavefront per 128-byte line it touches, and 32 lanes
-// stand at 32 places of their rows.  S lanes can share a target and read S
-// consecutive entries, which mostly lie in one cell: 16.8 lines a request with
-// S = 1 on the jittered Orszag-Tang slab, 11.9 with S = 2, 9.0 with S = 4.
-// Against that stand S times the per-target work (records, reductions, FP64
-// epilogue).  Force pass, S = 1 / 2 / 4: FP32 1 M slab 0.639 / 0.695 / 0.768 ms,
-// FP32 2 M Brio-Wu particles 0.862 / 1.008 / 1.213; FP64 206 k slab 0.393 / 0.327
-// / 0.317, FP64 176 k Brio-Wu 0.252 / 0.227 / 0.236.  So one lane in FP32, two
-// in FP64 (twice the bytes per record and fewer resident warps).
+// request costs the L1 about one wavefront per 128-byte line it touches, and 32
+// lanes stand at 32 places of their rows (9.6 wavefronts a gather on the jittered
+// Orszag-Tang slab).  S lanes can share a target and read S consecutive entries,
+// which mostly lie in one cell and touch fewer lines.  Against that stand S times
+// the per-target work (records, reductions, FP64 epilogue).  S = 1 / 2, ms:
+//   FP32 force  1 M slab 0.579 / 0.697, 1.35 M Kelvin-Helmholtz 0.821 / 0.960,
+//               2 M Brio-Wu particles 0.759 / 0.917
+//   FP32 build and density sum, the same three: 0.692 / 0.739, 1.072 / 1.136,
+//               1.212 / 1.292
+//   FP64 force  206 k slab 0.329 / 0.314, 176 k Brio-Wu particles 0.195 / 0.191
+//   FP64 build and density sum, the same two: 0.315 / 0.297, 0.281 / 0.270
+// So one lane in FP32, two in FP64 (twice the bytes per record and fewer resident
+// warps).
 //
 // Precision: an FP32 lane sums its entries in blocks of 8 folded by TwoSum
 // (CompAcc); FP64 lanes sum plainly.  Lane sums are added in FP64.
@@ -647,11 +651,16 @@ namespace sph
         //! below them one lane per target leaves most warp slots empty and the pass
         //! waits for its longest row.  The fold of every block by every lane costs
         //! 8 x 8 instructions per sum and round, so the line lies lower the more sums
-        //! a pass has.  One lane -> eight, ms: density Sod 2.3 k 0.064 -> 0.051 (with
-        //! the neighbour build), 18 k 0.103 -> 0.090, 36 k 0.098 -> 0.090, Orszag-Tang
-        //! 37 k 0.085 -> 0.082, 66 k 0.111 -> 0.117; hydro force Sod 2.3 k 0.029 -> 0.015,
-        //! 18 k 0.031 -> 0.025, 36 k 0.033 -> 0.038; SPMHD force Orszag-Tang 6.4 k
-        //! 0.028 -> 0.020, 16 k 0.028 -> 0.035.
+        //! a pass has.  One lane -> eight, ms:
+        //!   density (with the neighbour build)  Sod 2.3 k 0.051 -> 0.043, 18 k 0.093 ->
+        //!     0.084, 36 k 0.090 -> 0.087; Orszag-Tang 26 k 0.083 -> 0.075, 37 k 0.085 ->
+        //!     0.081, 45 k 0.092 -> 0.092, 54 k 0.102 -> 0.104, 66 k 0.112 -> 0.117
+        //!   hydro force  Sod 2.3 k 0.023 -> 0.012, 18 k 0.027 -> 0.024, 22 k 0.028 ->
+        //!     0.025, 26 k 0.029 -> 0.031, 31 k 0.029 -> 0.033, 36 k 0.029 -> 0.037
+        //!   SPMHD force  Orszag-Tang 4 k 0.032 -> 0.020, 8.1 k 0.032 -> 0.024, 9.2 k
+        //!     0.032 -> 0.024, 10 k 0.031 -> 0.032, 12 k 0.032 -> 0.035, 16 k 0.031 -> 0.038
+        //! Each line (256, 128 and 64 targets for each of the 148 SMs) lies on the gaining
+        //! side of its change of sign: 45 k, 22 to 26 k and 9.2 to 10 k.
         constexpr uint32_t kWideDensity = 148 * 256, kWideHydro = 148 * 128, kWideMhd = 148 * 64;
 
         template<int K, typename T, int PH>

@@ -15,9 +15,11 @@
 //
 // A pass is bound by latency and launches, not by its bytes (8 B in, 8 B out per
 // key): tiles of a fixed 4096 keys gave 18 k keys 5 blocks (10 us a histogram,
-// 12 us a scatter).  rounds follows the key count: about 128 tiles up to kFewKeys
-// keys, where the scatter adds the tiles' counts itself and step (2) needs no
-// launch, then four tiles per SM, then 16 rounds.
+// 12 us a scatter).  rounds follows the key count, rounded down: up to kFewKeys
+// keys the key count over 128 tiles (128 to 256 tiles come of it, fewer below 32 k
+// keys), above that over four tiles per SM (513 to 1184 tiles until 16 rounds, the
+// most a tile takes).  Up to kFewTiles tiles (to 49,152 keys, and from 65,536 to
+// kFewKeys) the scatter adds the tiles' counts itself and step (2) needs no launch.
 #include "sph_launch.hpp"
 
 namespace sph

@@ -95,7 +95,7 @@ namespace sph
         fb[3] = mhd ? psi * inv2 : 0.0;
     }
 
-    //! Box of a density work item (boxes are sorted by activeBase).
+    //! Box of a neighbour-build work item (boxes are sorted by activeBase).
     __device__ __forceinline__ int boxOfWork(BoxDev const* boxes, uint32_t nbox, uint32_t q)
     {
         int lo = 0, hi = int(nbox) - 1;
@@ -103,21 +103,6 @@ namespace sph
         {
             int const mid = (lo + hi + 1) >> 1;
             if(boxes[mid].activeBase <= q)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        return lo;
-    }
-
-    //! Box of a global cell id (boxes are sorted by cellBase).
-    __device__ __forceinline__ int boxOfCell(BoxDev const* boxes, uint32_t nbox, uint32_t cell)
-    {
-        int lo = 0, hi = int(nbox) - 1;
-        while(lo < hi)
-        {
-            int const mid = (lo + hi + 1) >> 1;
-            if(boxes[mid].cellBase <= cell)
                 lo = mid;
             else
                 hi = mid - 1;
@@ -238,6 +223,7 @@ namespace sph
         BoxDev* boxes;
         //! Per box, 32 entries: stencil slot s -> image shift (o_x e_x, o_y e_y, o_z e_z, 0)
         //! with o = the slot's offsets in {-1, 0, 1} and e = the cell edges (exact products).
+        //! Read by the FP64 pair passes (FP32 works the shift out from the slot).
         D4* shift64;
         Master cur, alt;
         Derivs d;
@@ -251,7 +237,10 @@ namespace sph
         uint32_t* valsB;
         uint32_t* sortScratch;
         uint32_t* status; //!< kStatWords words
-        uint32_t* work;   //!< density work queue: next cell to hand out (zeroed before each launch)
+        //! Neighbour build's queue: next item to hand out.  kDriftKeys (every build) and
+        //! kDensity (every density pass) zero it, so one of them runs between two
+        //! neighbour launches; a second launch alone would find the queue empty.
+        uint32_t* work;
         uint32_t* kickDone; //!< kick blocks finished; the last one finalises the step and resets it
         uint32_t* activeTotal; //!< work items of all boxes (their current cells, both levels)
         int32_t support;       //!< kernel support in units of h
@@ -405,7 +394,6 @@ namespace sph
         cudaStream_t s);
     uint32_t partialBlocks(uint32_t n);
 
-    // ---- pair_kernels.cu
     // ---- neighbours.cu
     //! Accepted-pair counts and list rows of the current cells; countOnly only
     //! counts.  `variant` picks the launch shape (0 = default, densityVariants).
