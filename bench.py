@@ -775,7 +775,7 @@ def run_ours(args, rank, world):
         result["arms"] = {
             "same_config": False,
             "differences": [
-                "value: the full north-star step (AV, SPMHD, Dedner, adaptive h, periodic images, 3 pair passes); "
+                "value: the full step (AV, SPMHD, Dedner, adaptive h, periodic images, 3 pair passes); "
                 "the reference has none of these, so the reference arm runs its own step on the same boxes",
                 "reference_physics: this GPU on exactly the reference arm's step and pair set (same 512 boxes, "
                 "density + inviscid hydro, one constant h per box, no periodic images, 2 pair passes)",
