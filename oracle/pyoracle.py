@@ -25,11 +25,12 @@ _REF = None
 
 def build(ref: bool = True, ref_root: str | None = None):
     """Compile the oracle, and the reference harness when a reference checkout
-    is given (``ref_root`` or the REF_ROOT environment variable) and exists;
-    without one the harness is left as it is (prebuilt, or absent)."""
+    is given (``ref_root`` or the REF_ROOT environment variable) and holds the
+    reference's headers; without one (no such directory, or an empty one) the
+    harness is left as it is (prebuilt, or absent)."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
     root = ref_root or os.environ.get("REF_ROOT")
-    if ref and root and os.path.isdir(root):
+    if ref and root and os.path.isdir(os.path.join(root, "include", "spearhed")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF_ROOT={root}"], check=True)
 
 

@@ -246,3 +246,13 @@ def test_neighbour_counts_match_brute_force(oracle):
     brute = (r2 < R * R).sum(1)
     assert np.array_equal(counts, brute)
     assert pairs == brute.sum()
+
+
+@pytest.mark.parametrize("present", [False, True])
+def test_build_without_the_references_headers_leaves_the_harness_alone(oracle, tmp_path, present):
+    """A checkout directory that does not exist or is empty builds the oracle only."""
+    root = tmp_path / "checkout"
+    if present:
+        root.mkdir()
+    oracle.build(ref=True, ref_root=str(root))
+    oracle.orc()
